@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "csr_tile.cuh"
+#include "resident_cg.cuh"
 
 namespace piro {
 
@@ -1225,6 +1226,40 @@ __global__ void __launch_bounds__(kPT, 2) k_be_persistent(PArgs P)
     }
 }
 
+// The whole solve by one team of CTAs with z, p, q, d of their lines in shared
+// memory (resident_cg.cuh).
+template <int kK, bool kStreamA>
+__global__ void __launch_bounds__(kRcThreads, 1) k_be_resident(RcProblem P,
+                                                               unsigned long long *epoch, RcSlot *slots,
+                                                               DevState *st, long long spin_limit)
+{
+    extern __shared__ float4 s_own[];
+    __shared__ RcShared sh;
+    const RcTeam T{slots, epoch, (int)blockIdx.x, (int)gridDim.x, &st->bar_err, spin_limit};
+    RcResult R;
+    rc_solve<false, kK, kStreamA>(P, T, sh, s_own, R);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->p_status = R.ok ? R.status : PIRO_ERR_CUDA;
+        st->p_outer = R.outer;
+        st->p_inner = R.inner;
+        st->p_rel = R.rel;
+    }
+}
+
+// The instance for a run of at most `groups` groups.
+const void *be_resident_kernel(int groups, bool stream_alpha)
+{
+    switch (cdiv(groups, kRcThreads)) {
+    case 0:
+    case 1: return (const void *)k_be_resident<1, false>;
+    case 2: return (const void *)k_be_resident<2, false>;
+    case 3: return (const void *)k_be_resident<3, false>;
+    case 4:
+    case 5: return (const void *)(stream_alpha ? k_be_resident<5, true> : k_be_resident<5, false>);
+    default: return (const void *)(stream_alpha ? k_be_resident<kRcK, true> : k_be_resident<kRcK, false>);
+    }
+}
+
 // The Jacobi iterations of a learned sweep in one cooperative launch: flexible
 // CG (the k_fcg_* iteration above) resumed from the state the network-
 // preconditioned iterations left -- r, the last direction p in p0 and its
@@ -1531,6 +1566,12 @@ struct piro_be_solver {
     int fcg_res;        // k_fcg_persistent<true> fits at grid_p blocks with res_smem
     int64_t res_cells;  // resident variant: cells per block, 0 if it does not fit
     size_t res_smem;
+    int rc_team;        // k_be_resident: CTAs of the team, 0 if the problem does not fit on chip
+    const void *rc_kernel;
+    char *rc_mem;       // the rounds' number (256 bytes), the team's slots, the exchange buffer; alpha
+    size_t rc_bytes;    // without alpha
+    size_t rc_smem;
+    RcProblem rc_problem;
     cudaEvent_t pev0, pev1;
     double persist_ms;
     long long persist_launches;
@@ -1581,6 +1622,7 @@ static void be_free(piro_be_solver *s)
     cudaFree(s->ib_col);
     cudaFree(s->ib_val);
     cudaFree(s->beff);
+    cudaFree(s->rc_mem);
     cudaFree(s->dinv);
     cudaFree(s->x64);
     cudaFree(s->partials);
@@ -1738,6 +1780,47 @@ static int be_setup_persistent(piro_be_solver *s, bool allow_resident)
     const int64_t fgrid = (int64_t)nsm * per_sm_f;
     s->grid_fp = (unsigned)(fgrid < grid ? fgrid : grid);
     s->fcg_res = 0;
+    // k_be_resident: the whole state on chip
+    s->rc_team = 0;
+    if (allow_resident) {
+        // Half a group per thread, as far as there are SMs: the phases of an
+        // iteration cost more than a larger team's all-reduce.  B200, kernel
+        // ms per step at 192 / 256 / 512 / 1024 groups per CTA: 24^3 0.177 /
+        // 0.151 / 0.171 / 0.196, 48^3 0.241 / 0.247 / 0.265 / 0.274, 64^3
+        // 0.256 / 0.255 / 0.271 / 0.295.
+        const int most = std::min(nsm, kRcMaxTeam);
+        const int64_t lines = (int64_t)(s->ny - 2) * (s->nz - 2), gx = (s->nx + 1) / 4;
+        const int64_t want = cdiv(lines * gx, kRcThreads / 2);
+        int team = (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min<int64_t>(most, lines)));
+        bool stream = false;
+        RcProblem rp = rc_geometry(s->nx, s->ny, s->nz, team);
+        if (rc_fits(rp, false, stream)) {
+            const void *kern = be_resident_kernel(rp.groups, stream);
+            static DeviceOnce once;
+            int rc2 = device_once(once, dev, []() -> int {
+                for (int groups = kRcThreads; groups <= kRcGroups; groups += kRcThreads)
+                    for (bool sa : {false, true})
+                        PIRO_CUDA(cudaFuncSetAttribute(be_resident_kernel(groups, sa),
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
+                return PIRO_OK;
+            });
+            if (rc2) return rc2;
+            int per_sm_rc = 0;
+            s->rc_smem = rc_smem(rp, false, stream);
+            PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rc, kern, kRcThreads, s->rc_smem));
+            if (per_sm_rc >= 1) {
+                const size_t ex = rc_exchange_bytes(s->nx, s->ny, s->nz), comm = 256 + rc_slot_bytes(team);
+                s->rc_bytes = comm + ex;
+                PIRO_CUDA(cudaMalloc(&s->rc_mem, s->rc_bytes + (stream ? ex / 2 : 0)));
+                PIRO_CUDA(cudaMemsetAsync(s->rc_mem, 0, s->rc_bytes, s->stream));
+                rp.zx = reinterpret_cast<uint4 *>(s->rc_mem + comm);
+                rp.ax = stream ? reinterpret_cast<float4 *>(s->rc_mem + s->rc_bytes) : nullptr;
+                s->rc_problem = rp;
+                s->rc_kernel = kern;
+                s->rc_team = team;
+            }
+        }
+    }
     // resident variant: every block's r, d, q in shared memory, if they fit
     // with the same grid still co-resident
     s->res_cells = 0;
@@ -1964,7 +2047,7 @@ extern "C" int piro_be_inner_operator(piro_be_solver *s, int *kind)
     *kind = s->op_mf ? (s->persist ? 2 : 1) : 0;
     if (*kind == 2) {  // the resident variant, when its float4 paths are usable at solve time
         const bool al16 = ((reinterpret_cast<uintptr_t>(s->alpha) | reinterpret_cast<uintptr_t>(s->dinv)) & 15) == 0;
-        if (s->res_cells > 0 && al16 && s->N % 4 == 0 && s->nx % 4 == 0) *kind = 3;
+        if (s->rc_team > 0 || (s->res_cells > 0 && al16 && s->N % 4 == 0 && s->nx % 4 == 0)) *kind = 3;
     }
     return PIRO_OK;
 }
@@ -2026,9 +2109,31 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
         const bool res = s->res_cells > 0 && P.vec_a;
         P.own_cells = res ? s->res_cells : 0;
         void *args[] = {&P};
+        RcProblem Q = s->rc_problem;
+        unsigned long long *epoch = reinterpret_cast<unsigned long long *>(s->rc_mem);
+        RcSlot *slots = reinterpret_cast<RcSlot *>(s->rc_mem + 256);
+        void *rargs[] = {&Q, &epoch, &slots, &s->st, &P.spin_limit};
         PIRO_CUDA(cudaMemsetAsync(s->st, 0, sizeof(DevState), st));
         PIRO_CUDA(cudaEventRecord(s->pev0, st));
-        if (res)
+        if (s->rc_team > 0) {
+            Q.alpha = s->alpha;
+            Q.mdt = s->mdt;
+            Q.vself = s->vself;
+            Q.vnb = s->vnb;
+            Q.b = b;
+            Q.xout = x;
+            Q.x64 = s->x64;
+            Q.beff = s->beff;
+            Q.ib_ptr = s->ib_ptr;
+            Q.ib_col = s->ib_col;
+            Q.ib_val = s->ib_val;
+            Q.rtol = rtol;
+            Q.inner_floor = s->inner_floor;
+            Q.max_outer = max_outer;
+            Q.max_inner = max_inner;
+            PIRO_CUDA(cudaLaunchCooperativeKernel(s->rc_kernel, dim3(s->rc_team), dim3(kRcThreads), rargs,
+                                                  s->rc_smem, st));
+        } else if (res)
             PIRO_CUDA(cudaLaunchCooperativeKernel((const void *)k_be_persistent<true>, dim3(s->grid_p), dim3(kPT), args,
                                                   s->res_smem, st));
         else
@@ -2056,6 +2161,8 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
         if (s->h_st->bar_err) {
             piro::set_error("piro_be_solve: grid barrier timed out");
             inf.status = PIRO_ERR_CUDA;
+            // the rounds that slots and exchange buffer hold are not known
+            if (s->rc_team > 0) PIRO_CUDA(cudaMemsetAsync(s->rc_mem, 0, s->rc_bytes, st));
         }
         if (info) *info = inf;
         return inf.status;
