@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "resident_cg.cuh"
 
 namespace piro {
 namespace {
@@ -797,6 +798,97 @@ __global__ void __launch_bounds__(kThreads, 4) k_batch_groups(GArgs A)
     }
 }
 
+// ---------------------------------------------------------------------------
+// The grouped step on chip (k_batch_resident), for batches whose
+// backward-Euler members all fit: one CTA per SM, every member a job solved by
+// a team of CTAs with its whole Krylov state in shared memory and registers
+// (resident_cg.cuh).  The lockstep rounds stream every member from HBM once
+// per CG phase (256 members, 65 M cells: 33.5 ms, 54% of the HBM rate); here a
+// member passes through HBM a few times per step, and what is left is the
+// phases' shared-memory traffic and one all-reduce per iteration.  Teams are
+// contiguous runs of CTAs and every CTA takes its jobs in the order of the job
+// list, so that the first unfinished job of the list can always run.
+struct RJob {
+    RcProblem P;  // all but b and xout
+    int64_t off;
+    int member, gbase, gsize;
+    unsigned long long *epoch;
+    RcSlot *slots;
+};
+
+struct RArgs {
+    const BMember *mem;
+    const int *fe_tile_m;
+    const int64_t *fe_tile_s;
+    int nfe, tile;
+    const RJob *jobs;
+    const int *cta_ptr, *cta_jobs;  // CTA c works on jobs cta_jobs[cta_ptr[c] .. cta_ptr[c+1])
+    const float *u;
+    float *out;
+    BState *st;
+    BarrierState *bar;  // err: a wait ran out
+    double rtol, inner_floor;
+    int max_sweeps, max_inner;
+    long long spin_limit;
+};
+
+__global__ void __launch_bounds__(kRcThreads, 1) k_batch_resident(RArgs A)
+{
+    extern __shared__ float4 s_own[];
+    __shared__ RcShared sh;
+    __shared__ RJob J;
+    // forward-Euler members: one pass over their tiles by every CTA
+    for (int t = blockIdx.x; t < A.nfe; t += gridDim.x) {
+        const BMember m = A.mem[A.fe_tile_m[t]];
+        const int64_t s0 = A.fe_tile_s[t], s1 = min(s0 + (int64_t)A.tile, m.N);
+        const int64_t sxy = (int64_t)m.g.nx * m.g.ny;
+        const float *u = A.u + m.off;
+        float *o = A.out + m.off;
+        for (int64_t i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
+            const float c = u[i];
+            if (m.g.interior(i)) {
+                const float c2 = __fmul_rn(2.0f, c);
+                const float lx = __fsub_rn(__fadd_rn(u[i + 1], u[i - 1]), c2);
+                const float ly = __fsub_rn(__fadd_rn(u[i + m.g.nx], u[i - m.g.nx]), c2);
+                const float lz = __fsub_rn(__fadd_rn(u[i + sxy], u[i - sxy]), c2);
+                const float lap = __fadd_rn(__fadd_rn(lx, ly), lz);
+                o[i] = __fadd_rn(c, __fmul_rn(m.dt, __fmul_rn(m.alpha, lap)));
+            } else {
+                o[i] = c;
+            }
+        }
+    }
+#pragma unroll 1
+    for (int jj = A.cta_ptr[blockIdx.x]; jj < A.cta_ptr[blockIdx.x + 1]; ++jj) {
+        __syncthreads();  // the last job's use of J
+        const int *src = reinterpret_cast<const int *>(A.jobs + A.cta_jobs[jj]);
+        for (int i = threadIdx.x; i < (int)(sizeof(RJob) / sizeof(int)); i += kRcThreads) reinterpret_cast<int *>(&J)[i] = src[i];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            J.P.b = A.u + J.off;
+            J.P.xout = A.out + J.off;
+            J.P.rtol = A.rtol;
+            J.P.inner_floor = A.inner_floor;
+            J.P.max_outer = A.max_sweeps;
+            J.P.max_inner = A.max_inner;
+        }
+        __syncthreads();
+        const RcTeam T{J.slots, J.epoch, (int)blockIdx.x - J.gbase, J.gsize, &A.bar->err, A.spin_limit};
+        RcResult R;
+        rc_solve<true, kRcK, false, const RcProblem &>(J.P, T, sh, s_own, R);
+        if (T.rank == 0 && threadIdx.x == 0) {
+            BState s{};
+            s.mode = kDone;
+            s.status = R.status;
+            s.sweep = R.outer;
+            s.it = s.inner_total = R.inner;
+            s.rel = R.rel;
+            A.st[J.member] = s;
+        }
+        if (!R.ok) return;
+    }
+}
+
 }  // namespace
 }  // namespace piro
 
@@ -836,6 +928,10 @@ struct piro_batch {
     int *d_cta_ptr = nullptr, *d_cta_jobs = nullptr;
     unsigned *d_job_bar = nullptr;
     double *d_job_part = nullptr;
+    // the grouped step on chip (k_batch_resident): used when grouped = 1 and d_rjobs is set
+    RJob *d_rjobs = nullptr;
+    char *r_mem = nullptr;  // rounds, slots and exchange buffers of the jobs
+    size_t r_bytes = 0, r_smem = 0;
 };
 
 static void batch_free_groups(piro_batch *s)
@@ -849,8 +945,148 @@ static void batch_free_groups(piro_batch *s)
     s->d_cta_ptr = s->d_cta_jobs = nullptr;
     s->d_job_bar = nullptr;
     s->d_job_part = nullptr;
+    cudaFree(s->d_rjobs);
+    cudaFree(s->r_mem);
+    s->d_rjobs = nullptr;
+    s->r_mem = nullptr;
     s->njobs = 0;
     s->grid_g = 0;
+}
+
+// The jobs of k_batch_resident.  A member's team is at least the smallest one
+// that holds it: SM time is least there, since a CTA's share of the all-reduces
+// does not shrink with its cells.  Where the batch leaves SMs idle, larger
+// teams end sooner, so a few common factors are tried on the list schedule
+// below and the shortest is taken.  Cycles of an iteration from the 128^3
+// solve's phases (B200): 8000 for a team's waits (3000 for one CTA's), 3.5 per
+// group of a CTA.  Returns PIRO_OK with d_rjobs unset if a member does not fit.
+static int batch_resident_setup(piro_batch *s)
+{
+    int dev = 0;
+    PIRO_CUDA(cudaGetDevice(&dev));
+    static DeviceOnce once;
+    int rc = device_once(once, dev, []() -> int {
+        PIRO_CUDA(cudaFuncSetAttribute(k_batch_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
+        return PIRO_OK;
+    });
+    if (rc) return rc;
+    int per_sm = 0;
+    PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_resident, kRcThreads, kRcSmemMax));
+    if (per_sm < 1) return PIRO_OK;
+    const int C = std::min(sm_count(), kRcMaxTeam);
+    std::vector<int> be;
+    for (int k = 0; k < s->M; ++k)
+        if (s->mem[k].scheme == 1) be.push_back(k);
+    // q and d always in shared memory here: the kernel has one instance
+    auto smem_of = [](const RcProblem &P) {
+        return 16 * ((size_t)3 * P.groups + ((size_t)P.halo + 1) * P.gx) + 12 * (size_t)(P.groups / P.gx) +
+               4 * (size_t)P.halo + 64;
+    };
+    auto fits = [&](const RcProblem &P) { return P.groups <= kRcGroups && smem_of(P) <= kRcSmemMax; };
+    std::vector<int> least(be.size());
+    for (size_t i = 0; i < be.size(); ++i) {
+        const int n = s->mem[be[i]].g.nx, gx = (n + 1) / 4, lines = (n - 2) * (n - 2);
+        int g = gx <= kRcGroups ? (int)cdiv(lines, kRcGroups / gx) : C + 1;
+        while (g <= std::min(C, lines) && !fits(rc_geometry(n, n, n, g))) ++g;
+        if (g > std::min(C, lines)) return PIRO_OK;
+        least[i] = g;
+    }
+    std::vector<size_t> order(be.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = i;
+    std::sort(order.begin(), order.end(), [&](size_t a, size_t b) { return least[a] != least[b] ? least[a] > least[b] : a < b; });
+    struct Plan {
+        double end = INFINITY;
+        std::vector<int> base, size;  // by position in `order`
+    } best;
+    for (double f : {1.0, 1.15, 1.35, 1.6, 2.0, 3.0, 5.0, 8.0, 16.0, 40.0}) {
+        Plan p;
+        p.end = 0.0;
+        p.base.resize(be.size());
+        p.size.resize(be.size());
+        std::vector<double> busy(C, 0.0);  // when each CTA is free
+        for (size_t o = 0; o < order.size(); ++o) {
+            const int n = s->mem[be[order[o]]].g.nx, gx = (n + 1) / 4, lines = (n - 2) * (n - 2);
+            // not below half a group per thread (the single solve's rule), nor past the lines
+            const int most = std::max<int>(least[order[o]], (int)std::min<int64_t>({(int64_t)C, (int64_t)lines,
+                                                                                    cdiv((int64_t)lines * gx, kRcThreads / 2)}));
+            const int g = std::min(most, (int)std::ceil(least[order[o]] * f));
+            const double cost = (g > 1 ? 8000.0 : 3000.0) + 3.5 * (double)(cdiv(lines, g) * gx);
+            int at = 0;
+            double start = INFINITY;
+            for (int b = 0; b + g <= C; ++b) {
+                double t = 0.0;
+                for (int c = b; c < b + g; ++c) t = std::max(t, busy[c]);
+                if (t < start) {
+                    start = t;
+                    at = b;
+                }
+            }
+            for (int c = at; c < at + g; ++c) busy[c] = start + cost;
+            p.base[o] = at;
+            p.size[o] = g;
+            p.end = std::max(p.end, start + cost);
+        }
+        if (p.end < best.end) best = p;
+    }
+    std::vector<RJob> jobs(be.size());
+    std::vector<std::vector<int>> cta(C);
+    size_t bytes = 0;
+    s->r_smem = 0;
+    for (size_t o = 0; o < order.size(); ++o) {
+        RJob &J = jobs[o];
+        const BMember &m = s->mem[be[order[o]]];
+        J.member = be[order[o]];
+        J.gbase = best.base[o];
+        J.gsize = best.size[o];
+        J.off = m.off;
+        J.P = rc_geometry(m.g.nx, m.g.nx, m.g.nx, J.gsize);
+        if (!fits(J.P)) return PIRO_OK;  // a larger team's strips can need more halo: keep the other kernel
+        J.P.alpha0 = m.alpha;
+        J.P.mdt = -m.dt;
+        J.P.vself = -6.0f;
+        J.P.vnb = 1.0f;
+        J.P.cd64 = m.cd64;
+        J.P.co64 = m.co64;
+        J.P.x64 = s->x64 + m.off;
+        s->r_smem = std::max(s->r_smem, smem_of(J.P));
+        if (J.gsize > 1) {  // offsets for now
+            J.epoch = reinterpret_cast<unsigned long long *>(bytes);
+            J.slots = reinterpret_cast<RcSlot *>(bytes + 256);
+            J.P.zx = reinterpret_cast<uint4 *>(bytes + 256 + rc_slot_bytes(J.gsize));
+            bytes += 256 + rc_slot_bytes(J.gsize) + (size_t)cdiv((int64_t)rc_exchange_bytes(m.g.nx, m.g.nx, m.g.nx), 256) * 256;
+        }
+        for (int c = J.gbase; c < J.gbase + J.gsize; ++c) cta[c].push_back((int)o);
+    }
+    std::vector<int> ptr(C + 1, 0), list;
+    for (int c = 0; c < C; ++c) {
+        ptr[c] = (int)list.size();
+        list.insert(list.end(), cta[c].begin(), cta[c].end());
+    }
+    ptr[C] = (int)list.size();
+    cudaError_t e = cudaMalloc(&s->r_mem, bytes > 0 ? bytes : 256);
+    if (e == cudaSuccess) e = cudaMemset(s->r_mem, 0, bytes > 0 ? bytes : 256);
+    for (RJob &J : jobs)
+        if (J.gsize > 1) {
+            J.epoch = reinterpret_cast<unsigned long long *>(s->r_mem + reinterpret_cast<size_t>(J.epoch));
+            J.slots = reinterpret_cast<RcSlot *>(s->r_mem + reinterpret_cast<size_t>(J.slots));
+            J.P.zx = reinterpret_cast<uint4 *>(s->r_mem + reinterpret_cast<size_t>(J.P.zx));
+        }
+    auto up = [](void **dst, const void *src, size_t n) -> cudaError_t {
+        cudaError_t e2 = cudaMalloc(dst, n > 0 ? n : 8);
+        if (e2 == cudaSuccess && n > 0) e2 = cudaMemcpy(*dst, src, n, cudaMemcpyHostToDevice);
+        return e2;
+    };
+    if (e == cudaSuccess) e = up((void **)&s->d_cta_ptr, ptr.data(), ptr.size() * sizeof(int));
+    if (e == cudaSuccess) e = up((void **)&s->d_cta_jobs, list.data(), list.size() * sizeof(int));
+    if (e == cudaSuccess) e = up((void **)&s->d_rjobs, jobs.data(), jobs.size() * sizeof(RJob));
+    if (e != cudaSuccess) {
+        set_error("piro_batch: grouped step setup failed: %s", cudaGetErrorString(e));
+        return PIRO_ERR_CUDA;
+    }
+    s->r_bytes = bytes;
+    s->njobs = (int)jobs.size();
+    s->grid_g = (unsigned)C;
+    return PIRO_OK;
 }
 
 // Jobs of the grouped step for a grid of sm_count * blocks_per_sm CTAs: with
@@ -861,6 +1097,11 @@ static void batch_free_groups(piro_batch *s)
 static int batch_groups_setup(piro_batch *s, int blocks_per_sm)
 {
     batch_free_groups(s);
+    const int rc = batch_resident_setup(s);
+    if (rc || s->d_rjobs) {
+        if (rc) batch_free_groups(s);
+        return rc;
+    }
     int per_sm = 0;
     PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_groups, kThreads, 0));
     if (per_sm < 1) {
@@ -1068,6 +1309,7 @@ extern "C" int piro_batch_create(int count, const int *n, const float *alpha, co
         if (e == cudaSuccess) e = cudaMalloc(p, N * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&s->x64, N * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&s->st, sizeof(BState) * count);
+    if (e == cudaSuccess) e = cudaMemset(s->st, 0, sizeof(BState) * count);
     if (e == cudaSuccess) e = cudaMalloc(&s->bar, sizeof(BarrierState));
     if (e == cudaSuccess) e = cudaMemset(s->bar, 0, sizeof(BarrierState));
     for (float *p : {s->f[0], s->f[1], s->b, s->r, s->p0, s->p1, s->q, s->d})
@@ -1158,9 +1400,36 @@ static int batch_launch_groups(piro_batch *s, const float *u, float *out, cudaSt
     return PIRO_OK;
 }
 
+static int batch_launch_resident(piro_batch *s, const float *u, float *out, cudaStream_t st)
+{
+    RArgs A;
+    A.mem = s->d_mem;
+    A.fe_tile_m = s->d_fe_m;
+    A.fe_tile_s = s->d_fe_s;
+    A.nfe = s->nfe;
+    A.tile = s->tile;
+    A.jobs = s->d_rjobs;
+    A.cta_ptr = s->d_cta_ptr;
+    A.cta_jobs = s->d_cta_jobs;
+    A.u = u;
+    A.out = out;
+    A.st = s->st;
+    A.bar = s->bar;
+    A.rtol = s->rtol;
+    A.inner_floor = 1e-6;
+    A.max_sweeps = 20;
+    A.max_inner = 20000;
+    A.spin_limit = wait_limit(1ll << 22);  // ~2 s of polling per wait
+    void *args[] = {&A};
+    PIRO_CUDA(cudaMemsetAsync(s->bar, 0, sizeof(BarrierState), st));
+    PIRO_CUDA(cudaLaunchCooperativeKernel((const void *)k_batch_resident, dim3(s->grid_g), dim3(kRcThreads), args,
+                                          s->r_smem, st));
+    return PIRO_OK;
+}
+
 static int batch_launch(piro_batch *s, const float *u, float *out, cudaStream_t st)
 {
-    if (s->grouped) return batch_launch_groups(s, u, out, st);
+    if (s->grouped) return s->d_rjobs ? batch_launch_resident(s, u, out, st) : batch_launch_groups(s, u, out, st);
     BArgs A;
     A.mem = s->d_mem;
     A.M = s->M;
@@ -1255,6 +1524,8 @@ extern "C" int piro_batch_step(piro_batch *s, int steps, double rtol, double *ms
     PIRO_CUDA(cudaMemcpy(&hb, s->bar, sizeof(hb), cudaMemcpyDeviceToHost));
     if (hb.err) {
         set_error("piro_batch_step: grid barrier timed out");
+        // the rounds that slots and exchange buffers hold are not known
+        if (s->d_rjobs) PIRO_CUDA(cudaMemset(s->r_mem, 0, s->r_bytes > 0 ? s->r_bytes : 256));
         return PIRO_ERR_CUDA;
     }
     float t = 0.0f;
@@ -1318,6 +1589,7 @@ extern "C" int piro_batch_autotune(piro_batch *s, double rtol, int *tile_out, in
     for (int b : {2, 4}) {
         rc = batch_groups_setup(s, b);
         if (rc) return rc;
+        if (s->d_rjobs) b = 1;  // one CTA per SM, whatever is asked for
         s->grouped = 1;
         float ms = INFINITY;
         for (int rep = 0; rep < 2; ++rep) {
@@ -1336,9 +1608,10 @@ extern "C" int piro_batch_autotune(piro_batch *s, double rtol, int *tile_out, in
             best = ms;
             bg = b;
         }
+        if (s->d_rjobs) break;
     }
     if (bg) {
-        rc = batch_groups_setup(s, bg);
+        if (!s->d_rjobs) rc = batch_groups_setup(s, bg);
         if (rc) return rc;
         s->grouped = 1;
         bb = bg;

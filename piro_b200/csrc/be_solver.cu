@@ -1237,7 +1237,7 @@ __global__ void __launch_bounds__(kRcThreads, 1) k_be_resident(RcProblem P,
     __shared__ RcShared sh;
     const RcTeam T{slots, epoch, (int)blockIdx.x, (int)gridDim.x, &st->bar_err, spin_limit};
     RcResult R;
-    rc_solve<false, kK, kStreamA>(P, T, sh, s_own, R);
+    rc_solve<false, kK, kStreamA, const RcProblem>(P, T, sh, s_own, R);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->p_status = R.ok ? R.status : PIRO_ERR_CUDA;
         st->p_outer = R.outer;

@@ -259,8 +259,8 @@ __device__ __forceinline__ unsigned long long rc_get(const RcSlot *p, double &v)
 // a wait ran out (sh.ok is 1 on entry).  One copy of the code serves every
 // sum: what a launch executes has to come through the instruction cache, and
 // with 60 KB more of it a solve took 100 us longer.
-__device__ __noinline__ bool rc_allreduce(const RcTeam &T, RcShared &sh, int first, int n, unsigned long long tag,
-                                          double v0, double v1, double v2, double v3, bool sync)
+static __device__ __noinline__ bool rc_allreduce(const RcTeam &T, RcShared &sh, int first, int n, unsigned long long tag,
+                                                 double v0, double v1, double v2, double v3, bool sync)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (T.size + 31) >> 5;
 #pragma unroll
@@ -342,9 +342,10 @@ struct RcVec {
 // with their own value and the stencil's coefficient); else alpha per cell,
 // and the interior-boundary block of A from ib_*.  kK: groups per thread
 // (with at most kRcRegK, q and d fit in registers beside D, w and p).
-// kStreamA: alpha is read from ax in every iteration.
-template <bool kConst, int kK, bool kStreamA>
-__device__ __forceinline__ void rc_solve(const RcProblem P, const RcTeam T, RcShared &sh, float4 *smem, RcResult &R)
+// kStreamA: alpha is read from ax in every iteration.  Prob: the problem by
+// value (a kernel's parameter) or by reference (in shared memory).
+template <bool kConst, int kK, bool kStreamA, class Prob>
+__device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, float4 *smem, RcResult &R)
 {
     constexpr bool kReg = kK <= kRcRegK;
     const int tid = threadIdx.x, lane = tid & 31;
