@@ -152,6 +152,11 @@ int piro_csr_fe_step(int nx, int ny, int nz, const int32_t *rowptr, const int32_
  * for bit as memset + piro_csr_fe_step + piro_set_bc. */
 int piro_csr_fe_step_bc(int nx, int ny, int nz, const int32_t *rowptr, const int32_t *col, const float *val, float dt,
                         const float *u, const float *bc, float *out, piro_stream_t stream);
+/* `steps` steps of piro_csr_fe_step_bc from u0 (the time loop of src/solve.cpp:18-46
+ * for TIMESCHEME 11, bit for bit): the field after them is in buf0 (even) or buf1
+ * (odd number of steps); the other buffer is scratch.  bc may be u0 or NULL. */
+int piro_csr_fe_run_bc(int nx, int ny, int nz, const int32_t *rowptr, const int32_t *col, const float *val, float dt,
+                       const float *u0, const float *bc, float *buf0, float *buf1, int steps, piro_stream_t stream);
 
 /* SpMVCSR_I1.cl:12-36 (backward-Euler residual form): interior rows get
  * out[r] = u[r] - sum_k (dt*val[k])*u[col[k]]; boundary rows untouched. */

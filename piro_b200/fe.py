@@ -1,9 +1,10 @@
 """Forward-Euler time loops (TIMESCHEME 11) on the device, one Solve() per
 step as src/solve.cpp:18-46 runs them: a zero-filled result buffer, the
 SpMV + update over the interior (SpMVCSR.cl), then setBC restoring the face
-values saved at start-up -- all three in one kernel (piro_csr_fe_step_bc).  The per-step launches can be captured once in
-a CUDA graph and replayed (graph=True), which removes the host from the loop
-for small grids where a step is a few microseconds."""
+values saved at start-up -- all three in one kernel (piro_csr_fe_step_bc).  A
+run is one call (piro_csr_fe_run_bc): small grids take all their steps in one
+launch.  The per-step launches can also be captured once in a CUDA graph and
+replayed (graph=True, capture)."""
 from __future__ import annotations
 
 import torch
@@ -12,8 +13,11 @@ from . import ops
 
 
 class _Loop:
+    @property
+    def bc_idx(self) -> torch.Tensor:
+        return ops.face_lists(self.nx, self.ny, self.nz)[0]
+
     def _setup_bc(self, u0: torch.Tensor) -> None:
-        self.bc_idx, _ = ops.face_lists(self.nx, self.ny, self.nz)
         self.memD = u0.clone()  # face values at start-up (bc.cpp:31-32)
 
     def _step(self, u: torch.Tensor, out: torch.Tensor) -> None:
@@ -46,12 +50,12 @@ class _Loop:
         return replay
 
     def run(self, u0: torch.Tensor, steps: int, graph: bool = False) -> torch.Tensor:
+        if not graph:
+            u0 = u0.contiguous()
+            bufs = [torch.empty_like(u0), torch.empty_like(u0)]
+            return ops.csr_fe_run_bc(self.nx, self.ny, self.nz, self.A, self.dt, u0, u0, *bufs, steps)
         self._setup_bc(u0)
         bufs = [u0.clone(), torch.empty_like(u0)]
-        if not graph:
-            for s in range(steps):
-                self._step(bufs[s & 1], bufs[(s + 1) & 1])
-            return bufs[steps & 1]
         # two steps per graph (buffers ping-pong), replayed steps//2 times
         stream = torch.cuda.Stream()
         stream.wait_stream(torch.cuda.current_stream())

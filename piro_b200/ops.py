@@ -224,6 +224,13 @@ def csr_fe_step_bc(nx, ny, nz, A, dt, u, bc, out):
     return out
 
 
+def csr_fe_run_bc(nx, ny, nz, A, dt, u0, bc, buf0, buf1, steps):
+    """steps of csr_fe_step_bc from u0; returns the buffer with the result."""
+    check(lib().piro_csr_fe_run_bc(nx, ny, nz, _p(A[0]), _p(A[1]), _p(A[2]), float(dt), _p(u0), _p(bc), _p(buf0),
+                                   _p(buf1), int(steps), _stream()), "piro_csr_fe_run_bc")
+    return buf1 if steps & 1 else buf0
+
+
 def ht_row_order(N, ts):
     """Rows by the home slot of their keys (for ht_spmv(order=...))."""
     n = C.c_size_t()
