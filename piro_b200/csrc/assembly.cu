@@ -9,6 +9,8 @@
 // pattern, so there is no scan, and the "first occurrence of column c" rule is
 // decided locally from c's coordinates.  Rows are staged in shared memory per
 // block so that col/val/rows leave the SM as coalesced stores.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace piro {
@@ -251,12 +253,45 @@ int64_t grad_prefix_host(int64_t i, int axis, const Grid &g, int64_t N)
     return grad_prefix(i, (int)(rem - (int64_t)y * g.nx), y, z, axis, g);
 }
 
-__global__ void k_rowscale(int64_t nrows, const int32_t *__restrict__ rowptr, float *__restrict__ val,
-                           const float *__restrict__ s)
+// val[k] *= s[row(k)], a warp per 32 rows: their entries are one contiguous
+// segment, which the warp moves through shared memory with consecutive lanes
+// on consecutive entries while each lane scales its own row there.  Bound by
+// the stream of val.  A thread per row on global memory took 73 us at 128^3
+// (128 MB), this form 24 us (B200).  A segment beyond the stage, or row
+// pointers that do not ascend, are scaled in place by the rows' lanes.
+constexpr int kScaleWarps = 8;
+constexpr int kScaleCap = 32 * 8;
+
+__global__ void __launch_bounds__(kScaleWarps * 32) k_rowscale(int64_t nrows, const int32_t *__restrict__ rowptr,
+                                                              float *__restrict__ val, const float *__restrict__ s)
 {
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x) {
-        const float f = s[r];
-        for (int32_t k = rowptr[r]; k < rowptr[r + 1]; ++k) val[k] = __fmul_rn(val[k], f);
+    __shared__ float s_v[kScaleWarps][kScaleCap];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t nchunk = (nrows + 31) >> 5;
+    for (int64_t ch = (int64_t)blockIdx.x * kScaleWarps + w; ch < nchunk; ch += (int64_t)gridDim.x * kScaleWarps) {
+        const int64_t row = (ch << 5) + lane;
+        const bool live = row < nrows;
+        const int last = (int)(nrows - (ch << 5) < 32 ? nrows - (ch << 5) : 32) - 1;
+        const int32_t k0 = live ? rowptr[row] : 0, k1 = live ? rowptr[row + 1] : 0;
+        const float f = live ? s[row] : 0.0f;
+        const int32_t b = __shfl_sync(0xffffffffu, k0, 0), e = __shfl_sync(0xffffffffu, k1, last);
+        const bool inside = !live || (b <= k0 && k0 <= k1 && k1 <= e);
+        if (!__all_sync(0xffffffffu, inside && e - b <= kScaleCap)) {
+            for (int32_t k = k0; k < k1; ++k) val[k] = __fmul_rn(val[k], f);
+            continue;
+        }
+        float r[kScaleCap / 32];  // the lane's loads in flight together
+#pragma unroll
+        for (int i = 0; i < kScaleCap / 32; ++i)
+            if (lane + 32 * i < e - b) r[i] = val[b + lane + 32 * i];
+#pragma unroll
+        for (int i = 0; i < kScaleCap / 32; ++i)
+            if (lane + 32 * i < e - b) s_v[w][lane + 32 * i] = r[i];
+        __syncwarp();
+        for (int32_t k = k0 - b; k < k1 - b; ++k) s_v[w][k] = __fmul_rn(s_v[w][k], f);
+        __syncwarp();
+        for (int t = lane; t < e - b; t += 32) val[b + t] = s_v[w][t];
+        __syncwarp();
     }
 }
 
@@ -456,7 +491,8 @@ extern "C" int piro_csr_rowscale(int64_t nrows, const int32_t *rowptr, float *va
 {
     PIRO_ARG(nrows >= 0 && rowptr && val && s, "piro_csr_rowscale: bad arguments");
     if (nrows == 0) return PIRO_OK;
-    k_rowscale<<<grid_for(nrows, 256, 8), 256, 0, as_stream(stream)>>>(nrows, rowptr, val, s);
+    k_rowscale<<<(unsigned)std::min<int64_t>(cdiv(nrows, 32 * kScaleWarps), (int64_t)sm_count() * 8), kScaleWarps * 32, 0,
+                 as_stream(stream)>>>(nrows, rowptr, val, s);
     PIRO_CHECK_LAUNCH("k_rowscale");
     return PIRO_OK;
 }

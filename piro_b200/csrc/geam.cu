@@ -43,7 +43,7 @@ __device__ __forceinline__ int64_t block_inclusive_scan(int64_t v, int64_t *s_wa
     return v;
 }
 
-// Pass 1: per-chunk sums of a[0..n).
+// Pass 1: per-chunk sums of a[0..n), consecutive lanes on consecutive items.
 __global__ void __launch_bounds__(kScanThreads) k_scan_sums(int64_t n, const int32_t *__restrict__ a,
                                                             int64_t *__restrict__ sums)
 {
@@ -52,11 +52,19 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(int64_t n, const int
     int64_t v = 0;
 #pragma unroll
     for (int t = 0; t < kScanItems; ++t) {
-        const int64_t i = base + (int64_t)threadIdx.x * kScanItems + t;
+        const int64_t i = base + (int64_t)t * kScanThreads + threadIdx.x;
         if (i < n) v += a[i];
     }
-    v = block_inclusive_scan(v, s_warp);
-    if (threadIdx.x == blockDim.x - 1) sums[blockIdx.x] = v;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        v = s_warp[threadIdx.x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (threadIdx.x == 0) sums[blockIdx.x] = v;
+    }
 }
 
 // Pass 2: exclusive scan of the chunk sums, one block, carried across rounds.
@@ -78,27 +86,44 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_offsets(int64_t nb, int64
     }
 }
 
-// Pass 3: in-place inclusive scan of a[0..n) plus the chunk offset.
+// Pass 3: in-place inclusive scan of a[0..n) plus the chunk offset.  A warp
+// takes 128 consecutive items, 32 at a time with consecutive lanes on
+// consecutive items; the warps' totals are scanned once per block.
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(int64_t n, int32_t *__restrict__ a,
                                                              const int64_t *__restrict__ offs)
 {
     __shared__ int64_t s_warp[32];
-    const int64_t base = (int64_t)blockIdx.x * kScanChunk;
-    int64_t loc[kScanItems];
-    int64_t v = 0;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * kScanChunk + (int64_t)w * (32 * kScanItems) + lane;
+    int64_t loc[kScanItems], run = 0;
+#pragma unroll
+    for (int t = 0; t < kScanItems; ++t) loc[t] = base + 32 * t < n ? a[base + 32 * t] : 0;
 #pragma unroll
     for (int t = 0; t < kScanItems; ++t) {
-        const int64_t i = base + (int64_t)threadIdx.x * kScanItems + t;
-        loc[t] = i < n ? a[i] : 0;
-        v += loc[t];
-    }
-    int64_t run = block_inclusive_scan(v, s_warp) - v + offs[blockIdx.x];
 #pragma unroll
-    for (int t = 0; t < kScanItems; ++t) {
-        const int64_t i = base + (int64_t)threadIdx.x * kScanItems + t;
-        run += loc[t];
-        if (i < n) a[i] = (int32_t)run;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t v = __shfl_up_sync(0xffffffffu, loc[t], o);
+            if (lane >= o) loc[t] += v;
+        }
+        loc[t] += run;
+        run = __shfl_sync(0xffffffffu, loc[t], 31);
     }
+    if (lane == 31) s_warp[w] = run;
+    __syncthreads();
+    if (w == 0) {
+        int64_t v = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        s_warp[lane] = v;
+    }
+    __syncthreads();
+    const int64_t add = offs[blockIdx.x] + (w > 0 ? s_warp[w - 1] : 0);
+#pragma unroll
+    for (int t = 0; t < kScanItems; ++t)
+        if (base + 32 * t < n) a[base + 32 * t] = (int32_t)(loc[t] + add);
 }
 
 // Counts for csrgeam_1.cl: lenA + lenB + lenC (no dedup, csrgeam_1.cl:27-67).
@@ -258,45 +283,149 @@ __device__ __forceinline__ int row_union(const int32_t *__restrict__ ca, int na,
     return n;
 }
 
-__global__ void k_geam2_count(int64_t N, const int32_t *__restrict__ rpA, const int32_t *__restrict__ cA,
-                              const int32_t *__restrict__ rpB, const int32_t *__restrict__ cB,
-                              int32_t *__restrict__ rpD, int *__restrict__ err)
+// The number of distinct columns of row r; -1 above kUnionMax entries.
+__device__ __noinline__ int geam2_count_row(const int32_t *__restrict__ ca, int na, const int32_t *__restrict__ cb,
+                                               int nb)
 {
     int32_t u[kUnionMax];
+    return row_union(ca, na, cb, nb, u);
+}
+
+// A + beta B in one row: the columns in ascending order, each with its A
+// entries in storage order, then its B entries.
+__device__ __noinline__ void geam2_fill_row(const int32_t *__restrict__ cA, const float *__restrict__ vA, int32_t a0,
+                                               int32_t a1, float beta, const int32_t *__restrict__ cB,
+                                               const float *__restrict__ vB, int32_t b0, int32_t b1, int64_t d0,
+                                               int32_t *__restrict__ cD, float *__restrict__ vD)
+{
+    int32_t u[kUnionMax];
+    const int n = row_union(cA + a0, a1 - a0, cB + b0, b1 - b0, u);
+    for (int t = 0; t < n; ++t) {
+        const int32_t c = u[t];
+        float acc = 0.0f;
+        bool have = false;
+        for (int32_t a = a0; a < a1; ++a)
+            if (cA[a] == c) { acc = have ? __fadd_rn(acc, vA[a]) : vA[a]; have = true; }
+        for (int32_t b = b0; b < b1; ++b)
+            if (cB[b] == c) {
+                const float t2 = __fmul_rn(beta, vB[b]);
+                acc = have ? __fadd_rn(acc, t2) : t2;
+                have = true;
+            }
+        cD[d0 + t] = c;
+        vD[d0 + t] = acc;
+    }
+}
+
+// Both passes hold a row of at most kG2Reg entries in registers, read by its
+// own lane (a warp's 32 rows cover contiguous runs of A and B, which L1 serves
+// after the first touch, as in csr_tile.cuh), and compare every pair of its
+// columns once.  The filled rows leave through shared memory, a warp's 32 rows
+// being one contiguous segment of D, with consecutive lanes on consecutive
+// entries.  I - dt L at 128^3 (B200): count 47 -> 22 us, fill 147 -> 63 us
+// against the union in a thread-local array (local memory) with stores entry
+// by entry, which longer rows still take.  Staging the inputs in shared
+// memory too was slower (32 and 95 us): issue slots, not the streams.
+constexpr int kG2Warps = 8;
+constexpr int kG2CapD = 32 * 8;
+constexpr int kG2Reg = 8;
+
+// A row's columns, A's entries before B's; entries past its end get columns
+// that match nothing.  first: bit t set if no earlier entry has column c[t].
+__device__ __forceinline__ unsigned geam2_columns(const int32_t *__restrict__ cA, int32_t a0, int na,
+                                                  const int32_t *__restrict__ cB, int32_t b0, int nb,
+                                                  int32_t (&c)[kG2Reg])
+{
+    unsigned first = 0;
+#pragma unroll
+    for (int t = 0; t < kG2Reg; ++t) c[t] = t < na ? cA[a0 + t] : t < na + nb ? cB[b0 + t - na] : -1 - t;
+#pragma unroll
+    for (int t = 0; t < kG2Reg; ++t) {
+        bool dup = t >= na + nb;
+#pragma unroll
+        for (int q = 0; q < t; ++q) dup |= c[q] == c[t];
+        first |= dup ? 0u : 1u << t;
+    }
+    return first;
+}
+
+__global__ void __launch_bounds__(256) k_geam2_count(int64_t N, const int32_t *__restrict__ rpA,
+                                                     const int32_t *__restrict__ cA, const int32_t *__restrict__ rpB,
+                                                     const int32_t *__restrict__ cB, int32_t *__restrict__ rpD,
+                                                     int *__restrict__ err)
+{
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
-        const int n = row_union(cA + rpA[r], rpA[r + 1] - rpA[r], cB + rpB[r], rpB[r + 1] - rpB[r], u);
-        if (n < 0) { atomicExch(err, 1); rpD[r + 1] = 0; }
-        else rpD[r + 1] = n;
+        const int32_t a0 = rpA[r], b0 = rpB[r];
+        const int na = rpA[r + 1] - a0, nb = rpB[r + 1] - b0;
+        int n;
+        if (na >= 0 && nb >= 0 && na + nb <= kG2Reg) {
+            int32_t c[kG2Reg];
+            n = __popc(geam2_columns(cA, a0, na, cB, b0, nb, c));
+        } else {
+            n = geam2_count_row(cA + a0, na, cB + b0, nb);
+        }
+        if (n < 0) atomicExch(err, 1);
+        rpD[r + 1] = n < 0 ? 0 : n;
         if (r == 0) rpD[0] = 0;
     }
 }
 
-__global__ void k_geam2_fill(int64_t N, const int32_t *__restrict__ rpA, const int32_t *__restrict__ cA,
-                             const float *__restrict__ vA, float beta, const int32_t *__restrict__ rpB,
-                             const int32_t *__restrict__ cB, const float *__restrict__ vB,
-                             const int32_t *__restrict__ rpD, int32_t *__restrict__ cD, float *__restrict__ vD)
+__global__ void __launch_bounds__(kG2Warps * 32, 6) k_geam2_fill(int64_t N, const int32_t *__restrict__ rpA,
+                                                              const int32_t *__restrict__ cA,
+                                                              const float *__restrict__ vA, float beta,
+                                                              const int32_t *__restrict__ rpB,
+                                                              const int32_t *__restrict__ cB,
+                                                              const float *__restrict__ vB,
+                                                              const int32_t *__restrict__ rpD, int32_t *__restrict__ cD,
+                                                              float *__restrict__ vD)
 {
-    int32_t u[kUnionMax];
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t a0 = rpA[r], a1 = rpA[r + 1], b0 = rpB[r], b1 = rpB[r + 1];
-        const int n = row_union(cA + a0, a1 - a0, cB + b0, b1 - b0, u);
-        if (n < 0) continue;
-        const int64_t d0 = rpD[r];
-        for (int t = 0; t < n; ++t) {
-            const int32_t c = u[t];
-            float acc = 0.0f;
-            bool have = false;
-            for (int32_t a = a0; a < a1; ++a)
-                if (cA[a] == c) { acc = have ? __fadd_rn(acc, vA[a]) : vA[a]; have = true; }
-            for (int32_t b = b0; b < b1; ++b)
-                if (cB[b] == c) {
-                    const float t2 = __fmul_rn(beta, vB[b]);
-                    acc = have ? __fadd_rn(acc, t2) : t2;
-                    have = true;
+    __shared__ int32_t s_c[kG2Warps][kG2CapD];
+    __shared__ float s_v[kG2Warps][kG2CapD];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t nchunk = (N + 31) >> 5;
+    for (int64_t ch = (int64_t)blockIdx.x * kG2Warps + w; ch < nchunk; ch += (int64_t)gridDim.x * kG2Warps) {
+        const int64_t row = (ch << 5) + lane;
+        const bool live = row < N;
+        const int last = (int)(N - (ch << 5) < 32 ? N - (ch << 5) : 32) - 1;
+        const int32_t a0 = live ? rpA[row] : 0, b0 = live ? rpB[row] : 0;
+        const int na = live ? rpA[row + 1] - a0 : 0, nb = live ? rpB[row + 1] - b0 : 0;
+        const int32_t d0 = live ? rpD[row] : 0, d1 = live ? rpD[row + 1] : 0;
+        const int32_t sd0 = __shfl_sync(0xffffffffu, d0, 0), sd1 = __shfl_sync(0xffffffffu, d1, last);
+        // every row short, and the rows of D where a merge of this chunk puts them
+        bool ok = !live || (na >= 0 && nb >= 0 && na + nb <= kG2Reg && sd0 <= d0 && d0 <= d1 && d1 <= sd1);
+        ok = __all_sync(0xffffffffu, ok) && sd1 - sd0 <= kG2CapD;
+        if (ok) {
+            // an entry that is its column's first goes to the place its column
+            // has among the firsts, with its repeats added in storage order
+            int32_t c[kG2Reg];
+            float v[kG2Reg];
+            const unsigned first = geam2_columns(cA, a0, na, cB, b0, nb, c);
+#pragma unroll
+            for (int t = 0; t < kG2Reg; ++t)
+                v[t] = t < na ? vA[a0 + t] : t < na + nb ? __fmul_rn(beta, vB[b0 + t - na]) : 0.0f;
+            const bool good = !live || __popc(first) == d1 - d0;
+#pragma unroll
+            for (int t = 0; t < kG2Reg; ++t)
+                if (good && (first >> t & 1u)) {
+                    int place = d0 - sd0;
+                    float acc = v[t];
+#pragma unroll
+                    for (int q = 0; q < kG2Reg; ++q) {
+                        if (q != t) place += (first >> q & 1u) && c[q] < c[t];
+                        if (q > t && c[q] == c[t]) acc = __fadd_rn(acc, v[q]);
+                    }
+                    s_c[w][place] = c[t];
+                    s_v[w][place] = acc;
                 }
-            cD[d0 + t] = c;
-            vD[d0 + t] = acc;
+            ok = __all_sync(0xffffffffu, good);
+            if (ok)
+                for (int t = lane; t < sd1 - sd0; t += 32) {
+                    cD[sd0 + t] = s_c[w][t];
+                    vD[sd0 + t] = s_v[w][t];
+                }
+            __syncwarp();
         }
+        if (!ok && live) geam2_fill_row(cA, vA, a0, a0 + na, beta, cB, vB, b0, b0 + nb, d0, cD, vD);
     }
 }
 
@@ -383,7 +512,8 @@ extern "C" int piro_csrgeam2_fill(int64_t N, const int32_t *rpA, const int32_t *
                                   int32_t *cD, float *vD, piro_stream_t stream)
 {
     PIRO_ARG(N > 0 && rpA && cA && vA && rpB && cB && vB && rpD && cD && vD, "piro_csrgeam2_fill: null argument");
-    k_geam2_fill<<<grid_for(N, 128, 8), 128, 0, as_stream(stream)>>>(N, rpA, cA, vA, beta, rpB, cB, vB, rpD, cD, vD);
+    k_geam2_fill<<<grid_for(N, 32 * kG2Warps, 8), kG2Warps * 32, 0, as_stream(stream)>>>(N, rpA, cA, vA, beta, rpB, cB, vB,
+                                                                                        rpD, cD, vD);
     PIRO_CHECK_LAUNCH("k_geam2_fill");
     return PIRO_OK;
 }
