@@ -674,6 +674,517 @@ __global__ void __launch_bounds__(256) k_lupb_update(int64_t N, int64_t bw, int6
                 *band_at(band, W, bw, r0 + ty + 16 * m, c0 + tx + 16 * n) = acc[m][n];
 }
 
+// ---------------------------------------------------------------------------
+// The blocked factorization in one cooperative launch (k_lupb_factor), for
+// bands whose panel has at most kLuPanelRows rows (and of bandwidth 16 or
+// more).  Block 0 factors the panels one after another and carries the next
+// panel's columns in shared memory from panel to panel; the other blocks apply
+// a panel to the columns right of those while block 0 factors the next one.
+//
+// Panel: a thread has two neighbouring rows in registers, rotated by four
+// columns every four steps so that the loop stays short; the multipliers stay
+// in the row and move with it, which gives the next panels' Lp directly.  A
+// step has one barrier: every warp's best candidate (the maximum of the
+// magnitude's bits in two steps, the first row on a tie) leaves its row in
+// shared memory before it is known whether it wins, as does the row that the
+// exchange displaces, and after the barrier every thread finds the winner
+// itself.  A step is a chain of latencies: about 2100 cycles, of which the two
+// searches take 600, a thread's two divisions 400, the rows' way through shared
+// memory 400 and the barrier 100.  One row per thread (20 warps instead of 10)
+// takes the same 35 thousand cycles a panel, bound by issue instead; a loop
+// over single steps 44; the next step's search before the rest of the row's
+// update 37.
+//
+// Four warps of block 0 fetch the next panel's columns meanwhile and publish
+// the finished panel, so that neither the wait for the other blocks (24 thousand
+// cycles) nor the fence is on the rows' path.
+//
+// Columns: a block owns the strips of 8 columns s with 1 + s mod (blocks - 1)
+// equal to it, in every panel, so that it only waits for block 0 (a ready
+// counter) and block 0 only for the two strips it takes over next.  A strip's
+// 16 pivot rows are substituted by shuffles, then one pass applies the 16 steps
+// to the rows below in order.  The blocks also store the panel's multipliers
+// to the band: from the panel's threads, a row each, these stores alone cost
+// block 0 1300 cycles a step.
+//
+// Every element receives the operations of the column launches in their
+// order: the band, the multipliers and the pivots are the same bits.  At 24^3
+// (864 panels of 592 rows) 23.3 ms, against 74.6 by three launches per panel
+// with the panel in shared memory and three barriers a step; 12^3 2.1 against
+// 7.1, 24 x 24 x 6 5.9 against 18.3 (B200).  Block 0 per panel, in thousands of
+// cycles: the steps 35, Lp and the row order out 5, the next columns' pivot rows
+// 2 and update 10.  Waits are bounded.
+constexpr int kLuPanelRows = 736;  // 512 threads, with 128 registers each
+constexpr int kLuStrip = 8;
+constexpr int kLuHelp = 128;  // block 0's threads that fetch and publish
+constexpr int kLuLd = kLuNbMax + 1;
+constexpr int kLuShare = 8;  // rows of multipliers a block stores at a time
+constexpr int kLuThreads = kLuPanelRows / 2 + 16 + kLuHelp;  // two rows per thread, in whole warps
+constexpr int kLuPerms = 8;  // panels whose row order is kept
+
+struct LuSync {
+    unsigned ready;  // panels factored
+    unsigned urgent; // strips applied that are the next panel but one
+    unsigned done;   // blocks x panels applied
+    int timeout;
+};
+
+struct LuArgs {
+    int64_t N, bw, W;
+    double *band, *Lc, *Lp;
+    int32_t *piv;
+    int *perm;  // [kLuPerms][bw + 16]
+    int *err;
+    LuSync *sync;
+    long long spin_limit;
+};
+
+// Waits until *count >= want; false if it ran out.  The caller orders what
+// follows by a fence: an acquire per poll would empty L1 each time.
+__device__ __forceinline__ bool lu_poll(const LuArgs &A, const unsigned *count, unsigned want)
+{
+    long long spins = 0;
+    while (true) {
+        unsigned c;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+        if (c >= want) return true;
+        if (++spins > A.spin_limit || *((volatile int *)&A.sync->timeout)) {
+            atomicExch(&A.sync->timeout, 1);
+            return false;
+        }
+    }
+}
+
+// Thread 0 waits; the result in every thread.
+__device__ __forceinline__ bool lu_wait(const LuArgs &A, const unsigned *count, unsigned want, int *s_flag)
+{
+    if (threadIdx.x == 0) {
+        *s_flag = lu_poll(A, count, want) ? 1 : 0;
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    __syncthreads();
+    return *s_flag != 0;
+}
+
+// The pivot rows of two columns per warp, a lane per row, by the panel's unit
+// lower triangle s_lw: lane's row is lane % 16, u its entry in column c.
+__device__ __forceinline__ double lu_pivot_rows(double u, const double *s_lw, int nbp, int64_t c, int64_t j0, int64_t bw)
+{
+    const int lane = threadIdx.x & 31, i = lane & 15;
+    const int64_t over = c - j0 - 2 * bw;  // step k reaches column j0 + k + 2bw
+    const int kmin = over > 0 ? (int)over : 0;
+    const bool mine = i < nbp && in_band(bw, j0 + i, c);
+    double l[kLuNbMax - 1];
+#pragma unroll
+    for (int k = 0; k < kLuNbMax - 1; ++k) l[k] = s_lw[i * kLuLd + k];  // 0 at and right of the diagonal
+#pragma unroll
+    for (int k = 0; k < kLuNbMax - 1; ++k) {
+        const double uk = __shfl_sync(0xffffffffu, u, (lane & 16) + k);
+        if (mine && l[k] != 0.0 && k >= kmin) u = fma(-l[k], uk, u);
+    }
+    return u;
+}
+
+// Applies the panel at j0 to the columns c0 .. c0 + 7 (those up to the last
+// one the panel reaches).  s_lp[k][row]: the panel's multipliers.  s_perm[r]:
+// the position, before the panel, of the row that ends at position r.  A
+// position below the panel that an exchange touched ends with a row that stood
+// in the panel, so the panel's rows as they were (s_o) and as they end (s_u)
+// are read first, and every other entry is read and written by the same thread.
+__device__ __forceinline__ void lu_strip(const LuArgs &A, const int *s_perm, const double *s_lw, const double *s_lp,
+                                         int64_t j0, int nbp, int R, int64_t c0, double *s_o, double *s_u)
+{
+    const int64_t bw = A.bw, W = A.W;
+    const int ldl = (int)(bw + kLuNbMax);
+    const int64_t cmax = j0 + nbp - 1 + 2 * bw < A.N - 1 ? j0 + nbp - 1 + 2 * bw : A.N - 1;
+    const int col = threadIdx.x % kLuStrip, r0 = nbp + threadIdx.x / kLuStrip, rows = blockDim.x / kLuStrip;
+    const int64_t c = c0 + col;
+    double v[4], next[4];  // the entries of four passes over the rows
+    auto fetch = [&](int r) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int rm = r + m * rows;
+            next[m] = rm < R && c <= cmax && in_band(bw, j0 + rm, c) ? *band_at(A.band, W, bw, j0 + rm, c) : 0.0;
+        }
+    };
+    fetch(r0);
+    if (threadIdx.x < kLuNbMax * kLuStrip) {
+        const int i = threadIdx.x & 15, cc = threadIdx.x >> 4;
+        const int64_t cw = c0 + cc;
+        double o = 0.0, u = 0.0;
+        if (i < nbp && cw <= cmax) {
+            const int64_t src = j0 + s_perm[i];
+            if (in_band(bw, j0 + i, cw)) o = *band_at(A.band, W, bw, j0 + i, cw);
+            if (in_band(bw, src, cw)) u = *band_at(A.band, W, bw, src, cw);
+        }
+        s_o[i * kLuLd + cc] = o;
+        s_u[i * kLuLd + cc] = lu_pivot_rows(u, s_lw, nbp, cw, j0, bw);
+    }
+    __syncthreads();
+    if (c <= cmax) {
+        const int kmin = c - j0 - 2 * bw > 0 ? (int)(c - j0 - 2 * bw) : 0;
+        double u[kLuNbMax];
+#pragma unroll
+        for (int k = 0; k < kLuNbMax; ++k) u[k] = s_u[k * kLuLd + col];
+        const int i = threadIdx.x / kLuStrip;
+        if (i < nbp && in_band(bw, j0 + i, c)) *band_at(A.band, W, bw, j0 + i, c) = s_u[i * kLuLd + col];
+#pragma unroll 1
+        for (int r = r0; r < R; r += 4 * rows) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) v[m] = next[m];
+            fetch(r + 4 * rows);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const int rm = r + m * rows;
+                if (rm >= R) break;
+                const int from = s_perm[rm];
+                double acc = from != rm ? s_o[from * kLuLd + col] : v[m];
+#pragma unroll
+                for (int k = 0; k < kLuNbMax; ++k) {
+                    const double l = s_lp[k * ldl + rm];
+                    if (l != 0.0 && k >= kmin) acc = fma(-l, u[k], acc);
+                }
+                if (in_band(bw, j0 + rm, c)) *band_at(A.band, W, bw, j0 + rm, c) = acc;
+            }
+        }
+    }
+    __syncthreads();  // s_o, s_u
+}
+
+__global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
+{
+    extern __shared__ double s_dyn[];  // block 0: the next panel's columns, [bw + 32][17]; others: Lp
+    constexpr int ld = kLuLd;
+    __shared__ double s_o[kLuNbMax * ld], s_lw[kLuNbMax * ld];
+    __shared__ __align__(16) double s_u[kLuNbMax * (kLuNbMax + 2)];
+    __shared__ __align__(16) double s_row[2][32][kLuNbMax], s_cur[2][kLuNbMax];
+    __shared__ uint2 s_max[2][32];
+    __shared__ int2 s_win[2][32];
+    __shared__ int s_curid[2], s_perm[kLuPanelRows], s_piv[kLuNbMax];
+    __shared__ int s_flag, s_stop;
+    const int64_t N = A.N, bw = A.bw, W = A.W;
+    const int ldl = (int)(bw + kLuNbMax);
+    const int npan = (int)cdiv(N, kLuNbMax);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto rows_of = [&](int64_t j0, int nbp) {
+        const int64_t rmax = j0 + nbp - 1 + bw < N - 1 ? j0 + nbp - 1 + bw : N - 1;
+        return (int)(rmax - j0 + 1);
+    };
+    if (blockIdx.x > 0) {
+        const int nb = gridDim.x - 1;
+#pragma unroll 1
+        for (int pi = 0; pi < npan; ++pi) {
+            const int64_t j0 = (int64_t)pi * kLuNbMax;
+            const int nbp = (int)(N - j0 < kLuNbMax ? N - j0 : kLuNbMax), R = rows_of(j0, nbp);
+            if (!lu_wait(A, &A.sync->ready, (unsigned)pi + 1, &s_flag)) return;
+            if (*((volatile int *)A.err)) return;
+            const int64_t cmax = j0 + nbp - 1 + 2 * bw < N - 1 ? j0 + nbp - 1 + 2 * bw : N - 1;
+            const int64_t first = (j0 + 2 * kLuNbMax) / kLuStrip, last = cmax / kLuStrip;
+            // the first strip at or after `first` that this block owns
+            int64_t st = first + (((int64_t)blockIdx.x - 1 - first) % nb + nb) % nb;
+            const double *lp = A.Lp + (int64_t)pi * kLuNbMax * ldl;
+            if (tid < kLuNbMax) s_piv[tid] = tid < nbp ? __ldcg(A.piv + j0 + tid) - (int)j0 : 0;
+            if (st <= last) {
+                for (int r = tid; r < R; r += blockDim.x) {
+                    s_perm[r] = __ldcg(A.perm + (pi % kLuPerms) * ldl + r);
+#pragma unroll
+                    for (int k = 0; k < kLuNbMax; ++k) {
+                        const double l = __ldcg(lp + k * ldl + r);
+                        s_dyn[k * ldl + r] = l;
+                        if (r < kLuNbMax) s_lw[r * ld + k] = r < nbp && k < r ? l : 0.0;
+                    }
+                }
+                __syncthreads();
+#pragma unroll 1
+                for (; st <= last; st += nb) {
+                    lu_strip(A, s_perm, s_lw, s_dyn, j0, nbp, R, st * kLuStrip, s_o, s_u);
+                    if (tid == 0 && st < first + kLuNbMax / kLuStrip)
+                        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&A.sync->urgent) : "memory");
+                }
+            } else
+                __syncthreads();
+            // The band holds a multiplier where it was computed, which for a row that
+            // an exchange moved is not where it ends: a block's share of the rows.
+            if (tid < kLuShare * kLuNbMax) {
+                const int k = tid % kLuNbMax;
+                for (int r = (int)blockIdx.x - 1 + nb * (tid / kLuNbMax); r < R; r += nb * kLuShare) {
+                    int q = r;
+                    if (r < nbp || __ldcg(A.perm + (pi % kLuPerms) * ldl + r) != r)
+#pragma unroll 1
+                        for (int kk = nbp - 1; kk > k; --kk) {
+                            const int pk = s_piv[kk];
+                            if (q == kk) q = pk;
+                            else if (q == pk) q = kk;
+                        }
+                    if (k < nbp && k < r && q - k <= bw) *band_at(A.band, W, bw, j0 + q, j0 + k) = __ldcg(lp + (int64_t)k * ldl + r);
+                }
+            }
+            __syncthreads();
+            if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&A.sync->done) : "memory");
+        }
+        return;
+    }
+    // Barriers of block 0, each used once a panel and in this order: kFree (the
+    // rows have taken s_dyn's values, the helpers may fill it), kFilled (they
+    // have), kPub (the rows have written what the helpers publish).
+    constexpr int kRowsBar = 1, kFree = 2, kFilled = 3, kPub = 4, kHelpBar = 5;
+    const int all = blockDim.x, rows = all - kLuHelp, nwarp = rows >> 5;
+    auto sync_on = [](int id, int n) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); };
+    auto arrive_on = [](int id, int n) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); };
+    if (tid == 0) {
+        s_flag = 1;
+        s_stop = 0;
+    }
+    __syncthreads();
+    if (tid >= rows) {  // the helpers
+        const int ht = tid - rows, cc = ht % kLuNbMax, r0 = ht / kLuNbMax;
+        constexpr int dr = kLuHelp / kLuNbMax;
+        unsigned due = 0;  // strips that were the next panel but one, so far
+#pragma unroll 1
+        for (int pi = 0; pi < npan; ++pi) {
+            const int64_t j0 = (int64_t)pi * kLuNbMax, j1 = j0 + kLuNbMax;
+            sync_on(kFree, all);
+            if (pi + 1 < npan) {
+                // The next panel's columns, once the strips of the last panel are in
+                // them; and that panel's slot for its row order, once it is read.
+                if (ht == 0) {
+                    const int64_t cl = j0 - kLuNbMax + kLuNbMax - 1 + 2 * bw < N - 1 ? j0 - 1 + 2 * bw : N - 1;  // the last panel's last column
+                    const int64_t left = pi > 0 ? cl / kLuStrip - j1 / kLuStrip + 1 : 0;
+                    due += left > kLuNbMax / kLuStrip ? kLuNbMax / kLuStrip : left > 0 ? (unsigned)left : 0u;
+                    const unsigned old = pi + 1 >= kLuPerms ? (unsigned)(pi + 2 - kLuPerms) * (gridDim.x - 1) : 0u;
+                    const bool ok = lu_poll(A, &A.sync->urgent, due) && lu_poll(A, &A.sync->done, old);
+                    if (!ok) s_flag = 0;
+                    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                }
+                sync_on(kHelpBar, kLuHelp);
+                if (s_flag) {
+                    const int n = rows_of(j1, (int)(N - j1 < kLuNbMax ? N - j1 : kLuNbMax)) + kLuNbMax;
+                    const bool col = j1 + cc < N;
+                    int64_t at = kLuNbMax + cc - r0 + bw;  // c - r + bw of row r0
+                    const double *src = A.band + (j0 + r0) * W + at;
+                    double *dst = s_dyn + r0 * ld + cc;
+#pragma unroll 4
+                    for (int r = r0; r < n; r += dr) {
+                        if (col && at >= 0 && at <= 3 * bw)
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                             (unsigned)__cvta_generic_to_shared(dst)),
+                                         "l"(src)
+                                         : "memory");
+                        else
+                            *dst = 0.0;
+                        at -= dr;
+                        src += dr * (W - 1);
+                        dst += dr * ld;
+                    }
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                }
+            }
+            arrive_on(kFilled, all);
+            sync_on(kPub, all);
+            if (!s_flag) return;
+            if (ht == 0) {
+                __threadfence();
+                atomicExch(&A.sync->ready, s_stop ? 0x7fffffffu : (unsigned)pi + 1);  // stop: every waiter sees err
+            }
+            if (s_stop) return;
+        }
+        return;
+    }
+    {
+        const int n = rows_of(0, (int)(N < kLuNbMax ? N : kLuNbMax));
+        for (int idx = tid; idx < n * kLuNbMax; idx += rows) {
+            const int r = idx / kLuNbMax, cc = idx % kLuNbMax;
+            s_dyn[(r + kLuNbMax) * ld + cc] = cc < N && in_band(bw, r, cc) ? *band_at(A.band, W, bw, r, cc) : 0.0;
+        }
+    }
+    sync_on(kRowsBar, rows);
+#pragma unroll 1
+    for (int pi = 0; pi < npan; ++pi) {
+        const int64_t j0 = (int64_t)pi * kLuNbMax;
+        const int nbp = (int)(N - j0 < kLuNbMax ? N - j0 : kLuNbMax);
+        const int R = rows_of(j0, nbp);
+        const int p0 = 2 * tid;         // this thread's positions: p0, p0 + 1
+        double a[2][kLuNbMax];          // the rows there, from column 4 jg on and round
+        int rid[2] = {p0, p0 + 1};      // their positions before the panel
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int cc = 0; cc < kLuNbMax; ++cc) a[h][cc] = p0 + h < R ? s_dyn[(p0 + h + kLuNbMax) * ld + cc] : 0.0;
+        arrive_on(kFree, all);
+        bool singular = false;
+#pragma unroll 1
+        for (int jg = 0; jg < 4 && !singular; ++jg) {
+#pragma unroll
+            for (int sj = 0; sj < 4; ++sj) {
+                const int jj = 4 * jg + sj, par = jj & 1;
+                if (jj >= nbp || singular) break;
+                const int64_t j = j0 + jj;
+                const int span = (int)(N - 1 - j < bw ? N - 1 - j : bw);
+                // the pivot of the step's column among the positions [jj, jj + span]
+                unsigned long long bits[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double v = fabs(a[h][sj]);
+                    const bool cand = p0 + h >= jj && p0 + h <= jj + span && v > 0.0;  // a NaN is no candidate
+                    bits[h] = cand ? (unsigned long long)__double_as_longlong(v) : 0ull;
+                }
+                const bool w = bits[1] > bits[0];
+                const unsigned long long best = w ? bits[1] : bits[0];
+                const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
+                const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+                const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+                const int win = __ffs(__ballot_sync(0xffffffffu, hi == mh && lo == ml)) - 1;
+                auto put = [&](double *dst, const double *row) {
+#pragma unroll
+                    for (int cc = 0; cc < kLuNbMax; cc += 2)
+                        *reinterpret_cast<double2 *>(dst + cc) = make_double2(row[cc], row[cc + 1]);
+                };
+                if (lane == win) {
+                    s_max[par][warp] = make_uint2(mh, ml);
+                    s_win[par][warp] = make_int2(p0 + (w ? 1 : 0), w ? rid[1] : rid[0]);
+                    if (w) put(s_row[par][warp], a[1]);
+                    else put(s_row[par][warp], a[0]);
+                }
+                if (p0 == (jj & ~1)) {
+                    s_curid[par] = rid[sj & 1];  // jj and sj are even together
+                    put(s_cur[par], a[sj & 1]);
+                }
+                sync_on(kRowsBar, rows);
+                const uint2 wm = lane < nwarp ? s_max[par][lane] : make_uint2(0u, 0u);
+                const unsigned bh = __reduce_max_sync(0xffffffffu, wm.x);
+                const unsigned bl = __reduce_max_sync(0xffffffffu, wm.x == bh ? wm.y : 0u);
+                const int from = __ffs(__ballot_sync(0xffffffffu, wm.x == bh && wm.y == bl)) - 1;
+                if (bh == 0u && bl == 0u) {
+                    if (tid == 0) {
+                        A.piv[j] = (int32_t)j;
+                        if (atomicCAS(A.err, 0, 3) == 0) A.err[1] = (int)j;
+                        s_stop = 1;
+                    }
+                    singular = true;
+                    break;
+                }
+                const int2 won = s_win[par][from];  // the pivot's position and row
+                const int p = won.x;
+                if (tid == 0) A.piv[j] = (int32_t)(j0 + p);
+                const double *pr = s_row[par][from];
+                if (p != jj) {  // the exchange, of the multipliers too
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (p0 + h == jj || p0 + h == p) {
+                            rid[h] = p0 + h == jj ? won.y : s_curid[par];
+                            const double *src = p0 + h == jj ? pr : s_cur[par];
+#pragma unroll
+                            for (int cc = 0; cc < kLuNbMax; ++cc) a[h][cc] = src[cc];
+                        }
+                }
+                const double ps = pr[sj];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int t = p0 + h - jj;
+                    if (t > 0 && t <= span) {
+                        // a quotient 0 / ps would send its warp through the division's slow path
+                        double l = __longlong_as_double((__double_as_longlong(a[h][sj]) ^ __double_as_longlong(ps)) & (1ll << 63));
+                        if (a[h][sj] != 0.0) l = a[h][sj] / ps;
+                        a[h][sj] = l;
+                        A.Lc[j * bw + t - 1] = l;
+                    }
+                }
+                const double l0 = p0 > jj && p0 <= jj + span ? a[0][sj] : 0.0;
+                const double l1 = p0 + 1 > jj && p0 + 1 <= jj + span ? a[1][sj] : 0.0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (jg + q < 4) {  // columns still to come
+#pragma unroll
+                        for (int cc = 4 * q; cc < 4 * q + 4; ++cc)
+                            if (cc > sj) {
+                                const double u = pr[cc];
+                                if (l0 != 0.0) a[0][cc] = fma(-l0, u, a[0][cc]);
+                                if (l1 != 0.0) a[1][cc] = fma(-l1, u, a[1][cc]);
+                            }
+                    }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double first[4];
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) first[cc] = a[h][cc];
+#pragma unroll
+                for (int cc = 0; cc < kLuNbMax - 4; ++cc) a[h][cc] = a[h][cc + 4];
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) a[h][kLuNbMax - 4 + cc] = first[cc];
+            }
+        }
+        // Lp[k][r]: the multiplier of step k for the row that ends at position r
+        if (!singular) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = p0 + h;
+                if (r >= R) continue;
+                A.perm[(pi % kLuPerms) * ldl + r] = rid[h];
+                s_perm[r] = rid[h];
+                if (r < nbp) {
+#pragma unroll
+                    for (int cc = 0; cc < kLuNbMax; ++cc) {
+                        if (cc >= r && cc < nbp) *band_at(A.band, W, bw, j0 + r, j0 + cc) = a[h][cc];
+                        a[h][cc] = cc < r ? a[h][cc] : 0.0;
+                        s_lw[r * ld + cc] = a[h][cc];
+                    }
+                }
+                double *lp = A.Lp + (int64_t)pi * kLuNbMax * ldl + r;
+#pragma unroll
+                for (int k = 0; k < kLuNbMax; ++k) lp[k * ldl] = k < nbp ? a[h][k] : 0.0;
+            }
+        }
+        arrive_on(kPub, all);
+        sync_on(kFilled, all);
+        if (singular || !s_flag || pi + 1 >= npan) return;
+        // The next panel's columns: exchanged, their pivot rows substituted, the
+        // rows below updated by their threads.  Rows 16 .. of s_dyn become the
+        // next panel.
+        const int64_t j1 = j0 + kLuNbMax;  // nbp = 16 here
+        constexpr int ldu = kLuNbMax + 2;
+        if (tid < kLuNbMax * kLuNbMax) {
+            const int i = tid & 15, cc = tid >> 4;
+            const double u = lu_pivot_rows(s_dyn[s_perm[i] * ld + cc], s_lw, nbp, j1 + cc, j0, bw);
+            s_u[i * ldu + cc] = u;
+            if (j1 + cc < N && in_band(bw, j0 + i, j1 + cc)) *band_at(A.band, W, bw, j0 + i, j1 + cc) = u;
+        }
+        sync_on(kRowsBar, rows);
+        if (p0 >= nbp && p0 < R) {  // nbp is even
+            // a row below the panel that an exchange touched stood in it: rid < 16
+            const double *src0 = s_dyn + rid[0] * ld, *src1 = s_dyn + rid[1] * ld;
+#pragma unroll
+            for (int c0 = 0; c0 < kLuNbMax; c0 += 8) {
+                double acc[2][8];
+#pragma unroll
+                for (int cc = 0; cc < 8; ++cc) {
+                    acc[0][cc] = src0[c0 + cc];
+                    acc[1][cc] = src1[c0 + cc];
+                }
+#pragma unroll
+                for (int k = 0; k < kLuNbMax; ++k) {
+                    const bool n0 = a[0][k] != 0.0, n1 = a[1][k] != 0.0;
+#pragma unroll
+                    for (int cc = 0; cc < 8; cc += 2) {
+                        const double2 u = *reinterpret_cast<const double2 *>(&s_u[k * ldu + c0 + cc]);
+                        if (n0) acc[0][cc] = fma(-a[0][k], u.x, acc[0][cc]);
+                        if (n0) acc[0][cc + 1] = fma(-a[0][k], u.y, acc[0][cc + 1]);
+                        if (n1) acc[1][cc] = fma(-a[1][k], u.x, acc[1][cc]);
+                        if (n1) acc[1][cc + 1] = fma(-a[1][k], u.y, acc[1][cc + 1]);
+                    }
+                }
+                // row p0 + 1 = R, past the panel's last, is one of the rows that enter
+#pragma unroll
+                for (int cc = 0; cc < 8; ++cc) {
+                    s_dyn[p0 * ld + c0 + cc] = acc[0][cc];
+                    if (p0 + 1 < R) s_dyn[(p0 + 1) * ld + c0 + cc] = acc[1][cc];
+                }
+            }
+        }
+        sync_on(kRowsBar, rows);
+    }
+}
+
 // Solve with the factor (one block): y = b in FP64; per step ro the row
 // exchange and the Gauss transform y[ro+t] -= l(t) y[ro]; then x from U,
 // row by row from the last (each row a block-wide dot product over its at
@@ -723,8 +1234,8 @@ __global__ void __launch_bounds__(kPivThreads) k_lup_solve(int64_t N, int64_t bw
 
 // The solve by the same 16-row panels.  Lp holds, per panel of 16 steps
 // starting at j0, the multipliers as the panel's later exchanges see them
-// ([bw + 16][16] doubles per panel, row r = position j0 + r), built once per
-// factorization from Lc and the pivots.  The forward pass per panel: the 16
+// ([16][bw + 16] doubles per panel, column r = position j0 + r), written by
+// k_lupb_factor or built once per factorization from Lc and the pivots.  The forward pass per panel: the 16
 // exchanges on y, the unit lower triangle (one thread, steps in order), then
 // the rows below it (a thread per row, steps in order); the backward pass per
 // panel from the last: for each of its rows the dot product with the solved
@@ -742,7 +1253,7 @@ __global__ void k_lup_lw_from_lc(int64_t N, int64_t bw, const double *__restrict
          idx += (int64_t)gridDim.x * blockDim.x) {
         const int64_t pi = idx / (R * kLuSolveNb);
         const int64_t rem = idx - pi * R * kLuSolveNb;
-        const int r = (int)(rem / kLuSolveNb), k = (int)(rem - (int64_t)r * kLuSolveNb);
+        const int k = (int)(rem / R), r = (int)(rem - (int64_t)k * R);
         const int64_t j0 = pi * kLuSolveNb;
         const int nbp = (int)(N - j0 < kLuSolveNb ? N - j0 : kLuSolveNb);
         double v = 0.0;
@@ -797,7 +1308,7 @@ __global__ void __launch_bounds__(kPivThreads) k_lup_solve_panels(int64_t N, int
         }
         for (int t = threadIdx.x; t < P * P; t += blockDim.x) {
             const int i = t / P, k = t - i * P;
-            s_t[i][k] = (i < nbp && k < i) ? lw[i * P + k] : 0.0;
+            s_t[i][k] = (i < nbp && k < i) ? lw[k * R + i] : 0.0;
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -842,7 +1353,7 @@ __global__ void __launch_bounds__(kPivThreads) k_lup_solve_panels(int64_t N, int
         for (int64_t r = j0 + nbp + threadIdx.x; r <= rmax; r += blockDim.x) {
             double acc = y[r];
             for (int k = 0; k < nbp; ++k) {
-                const double l = lw[(r - j0) * P + k];
+                const double l = lw[k * R + (r - j0)];
                 if (l != 0.0 && s_y[k] != 0.0) acc = fma(-l, s_y[k], acc);
             }
             y[r] = acc;
@@ -923,7 +1434,7 @@ __global__ void __launch_bounds__(kPivThreads) k_lup_solve_ring(int64_t N, int64
         if (threadIdx.x < nbp) s_piv[threadIdx.x] = piv[j0 + threadIdx.x];
         for (int t = threadIdx.x; t < P * P; t += blockDim.x) {
             const int i = t / P, k = t - i * P;
-            s_t[i][k] = (i < nbp && k < i) ? lw[i * P + k] : 0.0;
+            s_t[i][k] = (i < nbp && k < i) ? lw[k * R + i] : 0.0;
         }
         __syncthreads();
         if (threadIdx.x == 0)
@@ -957,7 +1468,7 @@ __global__ void __launch_bounds__(kPivThreads) k_lup_solve_ring(int64_t N, int64
             sr = sr >= WS ? sr - WS : sr;
             double acc = *yr;
             for (int k = 0; k < nbp; ++k) {
-                const double l = lw[(r - j0) * P + k];
+                const double l = lw[k * R + (r - j0)];
                 if (l != 0.0 && s_y[k] != 0.0) acc = fma(-l, s_y[k], acc);
             }
             *yr = acc;
@@ -1022,10 +1533,202 @@ __global__ void __launch_bounds__(kPivThreads) k_lup_solve_ring(int64_t N, int64
     for (int64_t r = threadIdx.x; r < N; r += blockDim.x) x[r] = (float)y[r];
 }
 
+// The ring solve with what a panel needs from global memory in registers
+// before the panel starts: the multipliers of a thread's two rows (forward) or
+// the lane's part of U's row (backward), loaded while the panel before it is
+// in its serial part, so that no panel waits for memory.  Bound by that serial
+// part: 15 dependent multiply-adds by shuffles forward, 16 dependent FP64
+// divisions backward.  Same arithmetic in the same order as k_lup_solve_ring.
+// 864 panels of bandwidth 576 (24^3): 5.8 ms, against 15.9 in k_lup_solve_ring
+// (B200); per panel 5 thousand cycles forward (the exchanges and the triangle
+// 1.4, the rows 1.7, issuing the next panel's loads 1.8) and 9 backward (the
+// triangle 3.8, the dot products 2.8, the loads 1.8).
+constexpr int kPreThreads = 512;                   // 16 warps: one per row of a panel backward
+constexpr int kPreU = 40;                          // entries of U per lane
+constexpr int64_t kPreBw = (kPreU * 32 - kLuSolveNb) / 2;  // 632: U's part and two rows per thread fit
+
+__global__ void __launch_bounds__(kPreThreads, 1) k_lup_solve_pre(int64_t N, int64_t bw, int64_t W,
+                                                                  const double *__restrict__ band,
+                                                                  const double *__restrict__ Lp,
+                                                                  const int32_t *__restrict__ piv,
+                                                                  const float *__restrict__ b, double *__restrict__ y,
+                                                                  float *__restrict__ x)
+{
+    constexpr int P = kLuSolveNb;
+    extern __shared__ double s_ring[];
+    __shared__ double s_y[P], s_dot[P];
+    __shared__ double s_t[P][P + 1];
+    __shared__ int32_t s_piv[P];
+    const uint32_t WS = (uint32_t)(2 * bw + P);
+    auto slot = [WS](int64_t r) { return (uint32_t)r % WS; };  // rows < 2^31
+    auto wrap = [WS](uint32_t v) { return v >= WS ? v - WS : v; };
+    const int64_t R = bw + P;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t npan = cdiv(N, P);
+    for (int64_t r = tid; r < N && r < (int64_t)WS; r += kPreThreads) s_ring[r] = (double)b[r];
+    // forward
+    double l0[P], l1[P], tri = 0.0, enter = 0.0;
+    int32_t pv = 0;
+    auto fetch = [&](int64_t pi) {
+        const double *lw = Lp + pi * R * P;
+        const int64_t j0 = pi * P;
+        const int nbp = (int)(N - j0 < P ? N - j0 : P);
+        const int64_t n0 = j0 + P + tid < N && tid < bw ? 1 : 0, n1 = j0 + P + tid + kPreThreads < N && tid + kPreThreads < bw;
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            l0[k] = n0 ? lw[k * R + P + tid] : 0.0;
+            l1[k] = n1 ? lw[k * R + P + tid + kPreThreads] : 0.0;
+        }
+        if (tid < P * P) {
+            const int i = tid / P, k = tid % P;
+            tri = i < nbp && k < i ? lw[k * R + i] : 0.0;
+        }
+        if (tid < nbp) {
+            pv = piv[j0 + tid];
+            enter = j0 + tid + WS < N ? (double)b[j0 + tid + WS] : 0.0;
+        }
+    };
+    fetch(0);
+    uint32_t s0 = 0;  // slot of row j0
+#pragma unroll 1
+    for (int64_t pi = 0; pi < npan; ++pi) {
+        const int64_t j0 = pi * P;
+        const int nbp = (int)(N - j0 < P ? N - j0 : P);
+        if (tid < P * P) s_t[tid / P][tid % P] = tri;
+        if (tid < nbp) s_piv[tid] = pv;
+        __syncthreads();
+        if (warp == 0) {
+            // The exchanges in registers: lane i < P holds the panel's row i, lane P + k
+            // the row of step k's pivot, unless a lower lane holds that row.
+            const int at = lane < P ? lane : lane - P < nbp ? (int)(s_piv[lane - P] - j0) : lane - P;
+            const int home = __ffs(__match_any_sync(0xffffffffu, at)) - 1;  // the lane that holds row `at`
+            const uint32_t here = wrap(s0 + at);                            // at < bw + P < WS
+            const bool mine = home == lane && (lane >= P || lane < nbp);
+            double yi = mine ? s_ring[here] : 0.0;
+            unsigned ex = __ballot_sync(0xffffffffu, lane >= P && home != lane - P) >> P;
+#pragma unroll 1
+            for (; ex; ex &= ex - 1) {
+                const int k = __ffs(ex) - 1, p = __shfl_sync(0xffffffffu, home, P + k);
+                const double other = __shfl_sync(0xffffffffu, yi, lane == k ? p : k);
+                if (lane == k || lane == p) yi = other;
+            }
+            if (mine && lane >= P) s_ring[here] = yi;
+            if (lane >= P) yi = 0.0;
+            double l[P];
+#pragma unroll
+            for (int k = 0; k < P - 1; ++k) l[k] = lane > k && lane < nbp ? s_t[lane & (P - 1)][k] : 0.0;
+#pragma unroll
+            for (int k = 0; k < P - 1; ++k) {
+                const double yk = __shfl_sync(0xffffffffu, yi, k);
+                if (l[k] != 0.0 && yk != 0.0) yi = fma(-l[k], yk, yi);  // l is 0 at and right of the diagonal
+            }
+            if (lane < nbp) {
+                s_y[lane] = yi;
+                s_ring[wrap(s0 + lane)] = yi;
+            }
+        }
+        __syncthreads();
+        // rows below: positions P + tid (and + kPreThreads); nbp < P only in the last panel, which has none
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t r = j0 + P + tid + h * kPreThreads;
+            if (tid + h * kPreThreads < bw && r < N) {
+                double *yr = &s_ring[wrap(s0 + P + tid + h * kPreThreads)];
+                double acc = *yr;
+#pragma unroll
+                for (int k = 0; k < P; ++k) {
+                    const double l = h ? l1[k] : l0[k], yk = s_y[k];
+                    if (l != 0.0 && yk != 0.0) acc = fma(-l, yk, acc);
+                }
+                *yr = acc;
+            }
+        }
+        if (tid < nbp) {  // these rows leave, rows WS further on enter
+            y[j0 + tid] = s_y[tid];
+            if (j0 + tid + WS < N) s_ring[wrap(s0 + tid)] = enter;
+        }
+        if (pi + 1 < npan) fetch(pi + 1);
+        s0 = wrap(s0 + P);
+    }
+    __syncthreads();
+    // backward; the ring holds rows [j0, j0 + WS)
+    double u[kPreU];
+    int cnt = 0;  // this lane's entries of the row
+    auto fetch_u = [&](int64_t pi) {
+        const int64_t j0 = pi * P;
+        const int nbp = (int)(N - j0 < P ? N - j0 : P);
+        const int64_t r = j0 + warp, c0 = j0 + nbp + lane;
+        const int64_t cmax = r + 2 * bw < N - 1 ? r + 2 * bw : N - 1;
+        const double *ur = band + r * W + (bw - r);  // ur[c] = U(r, c)
+        cnt = warp < nbp && cmax >= c0 ? (int)((cmax - c0) / 32) + 1 : 0;
+#pragma unroll
+        for (int i = 0; i < kPreU; ++i) u[i] = i < cnt ? ur[c0 + 32 * i] : 0.0;
+        if (tid < P * P) {
+            const int i = tid / P, c = tid % P;
+            tri = i < nbp && c < nbp && c >= i && c - i <= 2 * bw ? band[(j0 + i) * W + (c - i + bw)] : 0.0;
+        }
+        if (tid < nbp) enter = y[j0 + tid];
+    };
+    {
+        const int64_t j0 = (npan - 1) * P;
+        fetch_u(npan - 1);
+        s0 = slot(j0);
+    }
+#pragma unroll 1
+    for (int64_t pi = npan - 1; pi >= 0; --pi) {
+        const int64_t j0 = pi * P;
+        const int nbp = (int)(N - j0 < P ? N - j0 : P);
+        if (tid < nbp) {  // row r + WS (solved) leaves, row r (forward result) enters
+            const int64_t ro = j0 + tid + WS;
+            double *at = &s_ring[wrap(s0 + tid)];
+            if (ro < N) y[ro] = *at;
+            *at = enter;
+        }
+        __syncthreads();
+        if (tid < P * P) s_t[tid / P][tid % P] = tri;  // warp 0 has left the last panel's triangle
+        double sum = 0.0;
+        uint32_t sc = wrap(s0 + nbp + lane);
+#pragma unroll
+        for (int i = 0; i < kPreU; ++i) {
+            if (i < cnt) sum = fma(u[i], s_ring[sc], sum);
+            sc = wrap(sc + 32);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0 && warp < nbp) s_dot[warp] = sum;
+        if (pi > 0) fetch_u(pi - 1);
+        __syncthreads();
+        if (warp == 0) {
+            // lanes P .. repeat lanes 0 .. P-1: a quotient of zeros there would send
+            // the whole warp through the division's slow path
+            const int i = (lane & (P - 1)) < nbp ? lane & (P - 1) : 0;
+            const double *t = s_t[i], diag = t[i];
+            double dot = s_dot[i], yi = s_ring[wrap(s0 + i)];
+            double tc = t[nbp - 1];
+#pragma unroll 1
+            for (int c = nbp - 1; c >= 0; --c) {
+                const double q = (yi - dot) / diag;  // every lane's; lane c's is x_c
+                const double xc = __shfl_sync(0xffffffffu, q, c);
+                if (i == c) yi = q;
+                const double now = tc;
+                if (c > 0) tc = t[c - 1];
+                if (i < c) dot = fma(now, xc, dot);
+            }
+            if (lane < nbp) s_ring[wrap(s0 + lane)] = yi;
+        }
+        s0 = s0 >= P ? s0 - P : s0 + WS - P;
+    }
+    __syncthreads();
+    for (int64_t r = tid; r < N && r < (int64_t)WS; r += kPreThreads) y[r] = s_ring[slot(r)];
+    __syncthreads();
+    for (int64_t r = tid; r < N; r += kPreThreads) x[r] = (float)y[r];
+}
+
 // Device layout of the factor buffer: band double[N][3bw+1], Lc double[N][bw],
-// y double[N] (the solve's workspace), piv int32[N], err int[2], Lw
-// double[bw + 16][16] (the blocked factorization's panel multipliers), Lp
-// double[ceil(N/16)][bw + 16][16] (the solve's panel multipliers).
+// y double[N] (the solve's workspace), piv int32[N], err int[2] and LuSync, Lw
+// double[bw + 16][16] (the launched panels' multipliers) or perm int[2][bw + 16]
+// (k_lupb_factor's exchanges), Lp double[ceil(N/16)][16][bw + 16] (the solve's
+// panel multipliers).
 struct LupLayout {
     int64_t W;
     size_t band, lc, y, piv, err, lw, lp, total;  // byte offsets
@@ -1142,7 +1845,54 @@ extern "C" int piro_ht_lu_factor(int64_t N, int64_t bw, const int64_t *keys, con
         if ((size_t)(bw + t) * (t + 1) * sizeof(double) <= 200 * 1024) nb = t;
     const char *ub = getenv("PIRO_LU_UNBLOCKED");
     if (ub && ub[0] == '1') nb = 0;
-    if (nb) {
+    // One launch where the panel's rows fit in block 0's registers and the panel
+    // reaches columns past the next one (bw >= 16); the launches below otherwise.
+    bool one_launch = nb == kLuNbMax && bw >= kLuNbMax && bw + kLuNbMax <= kLuPanelRows;
+    if (one_launch) {
+        LuArgs A;
+        A.N = N;
+        A.bw = bw;
+        A.W = W;
+        A.band = AB;
+        A.Lc = Lc;
+        A.Lp = reinterpret_cast<double *>(base + L.lp);
+        A.piv = piv;
+        A.perm = reinterpret_cast<int *>(base + L.lw);
+        A.err = err;
+        A.sync = reinterpret_cast<LuSync *>(base + L.err + 64);
+        A.spin_limit = wait_limit(1ll << 22);  // ~2 s of polling per wait
+        const int threads = (int)std::max<int64_t>(256, cdiv(bw + kLuNbMax, 64) * 32) + kLuHelp;  // the pivot rows take 256
+        const size_t smem = (size_t)(bw + 2 * kLuNbMax) * kLuLd * sizeof(double);
+        static DeviceOnce once;
+        int dev = 0, coop = 0, per_sm = 0;
+        PIRO_CUDA(cudaGetDevice(&dev));
+        int rc = device_once(once, dev, []() -> int {
+            PIRO_CUDA(cudaFuncSetAttribute(k_lupb_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (kLuPanelRows + kLuNbMax) * kLuLd * (int)sizeof(double)));
+            return PIRO_OK;
+        });
+        if (rc) return rc;
+        PIRO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lupb_factor, threads, smem));
+        one_launch = coop && per_sm >= 1;
+        if (one_launch) {
+            // a block per strip of the columns right of the next panel, one block per SM
+            const int64_t strips = cdiv(2 * bw, kLuStrip) + 1;
+            const unsigned grid = (unsigned)(1 + std::min<int64_t>(strips, sm_count() - 1));
+            PIRO_CUDA(cudaMemsetAsync(A.sync, 0, sizeof(LuSync), st));
+            void *args[] = {&A};
+            PIRO_CUDA(cudaLaunchCooperativeKernel((const void *)k_lupb_factor, dim3(grid), dim3(threads), args, smem, st));
+            LuSync h;
+            PIRO_CUDA(cudaMemcpyAsync(&h, A.sync, sizeof(LuSync), cudaMemcpyDeviceToHost, st));
+            PIRO_CUDA(cudaStreamSynchronize(st));
+            if (h.timeout) {
+                set_error("piro_ht_lu_factor: a wait between blocks timed out");
+                return PIRO_ERR_CUDA;
+            }
+        }
+    }
+    if (one_launch) {
+    } else if (nb) {
         double *Lw = reinterpret_cast<double *>(base + L.lw);
         const size_t smem = (size_t)(bw + nb) * (nb + 1) * sizeof(double);
         PIRO_CUDA(cudaFuncSetAttribute(k_lupb_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1178,6 +1928,7 @@ extern "C" int piro_ht_lu_factor(int64_t N, int64_t bw, const int64_t *keys, con
         set_error("piro_ht_lu_factor: singular matrix: column %d has no nonzero at or below the diagonal", herr[1]);
         return PIRO_ERR_ZERO_PIVOT;
     }
+    if (one_launch) return PIRO_OK;  // Lp is written
     const int64_t lp_items = cdiv(N, kLuSolveNb) * (bw + kLuSolveNb) * kLuSolveNb;
     k_lup_lw_from_lc<<<grid_for(lp_items, 256, 8), 256, 0, st>>>(N, bw, Lc, piv,
                                                                    reinterpret_cast<double *>(base + L.lp));
@@ -1204,6 +1955,17 @@ extern "C" int piro_ht_lu_solve(int64_t N, int64_t bw, void *band, size_t band_b
     } else if ((size_t)(2 * bw + kLuSolveNb) * sizeof(double) <= 160 * 1024 &&
                !(getenv("PIRO_LU_NO_RING") && getenv("PIRO_LU_NO_RING")[0] == '1')) {
         const size_t smem = (size_t)(2 * bw + kLuSolveNb) * sizeof(double);
+        // What a panel reads fits in registers (at most 1280 ring rows, 10 KB): 5.8 ms
+        // at bandwidth 576, 13824 rows, against 15.9 from memory, and 0.64 against
+        // 0.96 at 144, 1728 rows.
+        if (bw >= kLuSolveNb && bw <= kPreBw) {
+            k_lup_solve_pre<<<1, kPreThreads, smem, st>>>(N, bw, L.W, reinterpret_cast<const double *>(base + L.band),
+                                                          reinterpret_cast<const double *>(base + L.lp),
+                                                          reinterpret_cast<const int32_t *>(base + L.piv), b,
+                                                          reinterpret_cast<double *>(base + L.y), x);
+            PIRO_CHECK_LAUNCH("k_lup_solve_pre");
+            return PIRO_OK;
+        }
         PIRO_CUDA(cudaFuncSetAttribute(k_lup_solve_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_lup_solve_ring<<<1, kPivThreads, smem, st>>>(N, bw, L.W, reinterpret_cast<const double *>(base + L.band),
                                                        reinterpret_cast<const double *>(base + L.lp),
