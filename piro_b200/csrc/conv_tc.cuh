@@ -3,27 +3,34 @@
 // the 5th-generation tensor cores: tcgen05.mma (kind::f16, BF16 operands,
 // FP32 accumulation in tensor memory), operands staged by TMA.
 //
-// Activations are channels-last BF16, 16 channels = 32 bytes per cell, on the
-// ghost-inclusive grid; boundary cells hold zeros.  An output tile is 128
-// consecutive cells (MMA M = 128), N = 16 output channels, and the K loop is
-// the 27 taps x 16 input channels: 27 MMAs of K = 16.
+// Activations are BF16 in two planes of 8 channels, [plane 2][cell][8], 16 bytes
+// per cell and plane, on the ghost-inclusive grid; boundary cells hold zeros.
+// A plane has act_rows(cells) rows: whole blocks of 8, and 8 more, zeros from
+// the last cell on.  An output tile is 128 consecutive cells (MMA M = 128),
+// N = 16 output channels, and the K loop is the 27 taps x 16 input channels:
+// 27 MMAs of K = 16.
 //
 // Operand A of tap (dx, dy, dz) is the input at rows c0 + dx + dy*nx + dz*nx*ny
-// + [0, 128).  For each (dy, dz) one "line block" of 130 rows (the tile and one
-// row each side) is loaded once; the three dx taps read it at row offsets 0, 1,
-// 2.  The line block sits in shared memory in the no-swizzle K-major layout of
-// the MMA -- [channel group 2][130 rows][8 channels], so an 8-row x 16-byte core
-// matrix is 128 contiguous bytes, consecutive rows are 16 bytes apart (SBO =
-// 128 bytes per 8 rows) and the two channel groups LBO = 130*16 bytes apart --
-// and a row offset is a 16-byte move of the descriptor's start address.  TMA
-// writes exactly that layout from a 3-D view of the activations:
-// (8 channels, rows with a 32-byte stride, 2 groups with a 16-byte stride),
-// box {8, 130, 2}.  Rows outside the array read as zeros (TMA fill).
+// + [0, 128).  For each (dy, dz) one "line block" of 136 rows (the tile, one row
+// before it and 7 after) is loaded once; the three dx taps read it at row
+// offsets 0, 1, 2.  The line block sits in shared memory in the no-swizzle
+// K-major layout of the MMA -- [channel group 2][136 rows][8 channels], so an
+// 8-row x 16-byte core matrix is 128 contiguous bytes, consecutive rows are 16
+// bytes apart (SBO = 128 bytes per 8 rows) and the two channel groups
+// LBO = 136*16 bytes apart -- and a row offset is a 16-byte move of the
+// descriptor's start address.
+//
+// TMA writes that layout in 128-byte pieces of 8 rows from a 4-D view of the
+// planes: (8 rows x 8 channels, first row 0..7 at 16 bytes, blocks of 8 rows,
+// planes), box {64, 1, 17, 2} at (0, r mod 8, floor(r / 8), 0) for first row r.
+// Blocks outside the planes read as zeros (TMA
+// fill): before the array and after it there are at least 13 boundary cells,
+// so the part of a block that lies in the array holds zeros too.
 //
 // A CTA owns one 128-cell column and marches it along z: the 9 line blocks of
 // tile z are the 3 of each of the planes z-1, z, z+1, so each new tile loads 3
 // line blocks (one plane) while the others stay resident: a ring of 4 planes
-// (3 in use, 1 loading).  L2 -> SM traffic is about 3 * 130/128 * 32 bytes
+// (3 in use, 1 loading).  L2 -> SM traffic is about 3 * 136/128 * 32 bytes
 // per output cell, against 27 * 32 for a load per tap.
 //
 // Batched grids (blockIdx.y = member b) are consecutive in the array: rows
@@ -50,11 +57,10 @@ namespace tc {
 typedef __nv_bfloat16 bf16;
 
 constexpr int kRows = 128;                    // output cells per tile (MMA M)
-constexpr int kLineRows = kRows + 2;          // rows of a line block
-constexpr int kLineBytes = kLineRows * 32;    // 4160
-constexpr int kLineStride = 4224;             // 128-byte aligned slot of a line block
+constexpr int kLineRows = kRows + 8;          // rows of a line block
+constexpr int kLineBytes = kLineRows * 32;    // 4352: a multiple of 128, as TMA wants
 constexpr int kSlots = 4;                     // planes resident (3 read by a tile, 1 loading)
-constexpr int kPlaneBytes = 3 * kLineStride;  // the 3 line blocks (dy = -1, 0, 1) of a plane
+constexpr int kPlaneBytes = 3 * kLineBytes;  // the 3 line blocks (dy = -1, 0, 1) of a plane
 constexpr int kWBytes = 27 * 512;             // one layer's weights: per tap [group][co 16][8 ci] BF16
 constexpr int kThreads = 192;
 constexpr int kBarOff = kSlots * kPlaneBytes + kWBytes;
@@ -62,6 +68,9 @@ constexpr int kAcc = 2;                       // TMEM accumulators (16 columns e
 constexpr int kBarSlots = 2 * kSlots + 2 * kAcc + 1;  // full, empty, acc_full, acc_empty, drain
 constexpr int kSmemBytes = kBarOff + kBarSlots * 8 + 16 + 128;  // + barriers, TMEM address, alignment slack
 constexpr long long kSpin = 1ll << 24;        // polls before a wait gives up
+
+// Rows of a plane of an activation array: the stride of its 8-row blocks divides it.
+__host__ __device__ inline int64_t act_rows(int64_t cells) { return (cells + 7) / 8 * 8 + 8; }
 
 struct Args {
     GridDiv g;
@@ -74,6 +83,7 @@ struct Args {
     double n_int;
     const int *skip;   // launch returns at once when set (may be NULL)
     int *err;          // raised on a timed-out wait
+    int64_t cells, rows;  // cells of the whole array, rows of a plane of 8 channels
     bf16 *yout;        // epilogue 2: the pre-activation bf16(acc)
     const bf16 *yprev; // epilogue 3: the previous layer's pre-activation
 };
@@ -125,12 +135,20 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity)
         if (mbar_try_wait(bar, parity)) return;
 }
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2)
+// The line block of both planes whose first row is r.
+__device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap *map, uint32_t bar, int64_t r)
 {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %3}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(0), "r"((int)(r & 7)), "r"((int)(r >> 3))
         : "memory");
+}
+
+// One cell's 16 channels, the planes' rows apart.
+__device__ __forceinline__ void put_cell(bf16 *act, int64_t rows, int64_t c, uint4 lo, uint4 hi)
+{
+    *reinterpret_cast<uint4 *>(act + c * 8) = lo;
+    *reinterpret_cast<uint4 *>(act + (rows + c) * 8) = hi;
 }
 
 // Shared-memory matrix descriptor, K-major, no swizzle: start address, LBO
@@ -266,8 +284,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                     mbar_expect_tx(full(slot), 3 * kLineBytes);
                     for (int dy = 0; dy < 3; ++dy) {
                         const int64_t r = boff + L * a.nxy + (int64_t)col * kRows - 1 + (int64_t)(dy - 1) * a.g.nx;
-                        tma_load_3d(planes_s + slot * kPlaneBytes + dy * kLineStride, &xmap, full(slot), 0, (int)r,
-                                    0);
+                        tma_load_rows(planes_s + slot * kPlaneBytes + dy * kLineBytes, &xmap, full(slot), r);
                     }
                 }
                 // no copy may land after the CTA has left, whatever the other
@@ -297,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                             for (int dx = 0; dx < 3; ++dx) {
                                 const int tap = dz * 9 + dy * 3 + dx;
                                 const uint64_t ad =
-                                    desc_nosw(pbase + dy * kLineStride + dx * 16, kLineRows * 16, 128);
+                                    desc_nosw(pbase + dy * kLineBytes + dx * 16, kLineRows * 16, 128);
                                 const uint64_t bd = desc_nosw(w_s + tap * 512, 256, 128);
                                 mma_bf16(d_tmem, ad, bd, tap > 0 ? 1u : 0u);
                             }
@@ -321,16 +338,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                 if (kEpi == 1) {
                     a.zout[boff + c] = 0.0f;
                 } else {
-                    uint4 *o = reinterpret_cast<uint4 *>(a.out + (boff + c) * 16);
-                    o[0] = make_uint4(0, 0, 0, 0);
-                    o[1] = make_uint4(0, 0, 0, 0);
-                    if (kEpi == 2) {
-                        uint4 *oy = reinterpret_cast<uint4 *>(a.yout + (boff + c) * 16);
-                        oy[0] = make_uint4(0, 0, 0, 0);
-                        oy[1] = make_uint4(0, 0, 0, 0);
-                    }
+                    const uint4 z4 = make_uint4(0, 0, 0, 0);
+                    put_cell(a.out, a.rows, boff + c, z4, z4);
+                    if (kEpi == 2) put_cell(a.yout, a.rows, boff + c, z4, z4);
                 }
             }
+            // and so do the rows after the last cell (the next layer's loads read them)
+            if (kEpi != 1 && warp == 0 && boff + a.N == a.cells && ze == a.g.nz - 1 && col == a.ncol - 1 &&
+                a.cells + lane < a.rows)
+                put_cell(a.out, a.rows, a.cells + lane, make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0));
             // epilogue: warp w holds tile rows 32w .. 32w+31
             for (int j = 0; j < P; ++j) {
                 const int buf = j % kAcc;
@@ -352,8 +368,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                     if (c < a.N) {
                         uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
                         if (a.g.interior(c)) {
-                            const uint4 *yp = reinterpret_cast<const uint4 *>(a.yprev + (boff + c) * 16);
-                            const uint4 u0 = yp[0], u1 = yp[1];
+                            const uint4 u0 = *reinterpret_cast<const uint4 *>(a.yprev + (boff + c) * 8);
+                            const uint4 u1 = *reinterpret_cast<const uint4 *>(a.yprev + (a.rows + boff + c) * 8);
                             const uint32_t yw[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
 #pragma unroll
                             for (int k = 0; k < 8; ++k) {
@@ -363,9 +379,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                                 w[k] = *reinterpret_cast<const uint32_t *>(&h);
                             }
                         }
-                        uint4 *o = reinterpret_cast<uint4 *>(a.out + (boff + c) * 16);
-                        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                        put_cell(a.out, a.rows, boff + c, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
                     }
                 } else if (c < a.N) {
                     uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, yw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -382,14 +396,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                             }
                         }
                     }
-                    uint4 *o = reinterpret_cast<uint4 *>(a.out + (boff + c) * 16);
-                    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
-                    if (kEpi == 2) {
-                        uint4 *oy = reinterpret_cast<uint4 *>(a.yout + (boff + c) * 16);
-                        oy[0] = make_uint4(yw[0], yw[1], yw[2], yw[3]);
-                        oy[1] = make_uint4(yw[4], yw[5], yw[6], yw[7]);
-                    }
+                    put_cell(a.out, a.rows, boff + c, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
+                    if (kEpi == 2)
+                        put_cell(a.yout, a.rows, boff + c, make_uint4(yw[0], yw[1], yw[2], yw[3]),
+                                 make_uint4(yw[4], yw[5], yw[6], yw[7]));
                 }
             }
         }

@@ -10,7 +10,8 @@
 // of the ghost-inclusive grid hold zero activations, so an interior cell's
 // 27 neighbours are always inside the array).  BF16 weights and activations,
 // FP32 accumulation.  Activations are stored channels-last (16 bf16 = 32 bytes
-// per cell); the output is FP32.
+// per cell) by the CUDA-core layers and in two planes of 8 channels by the
+// tensor-core layers (conv_tc.cuh); the output is FP32.
 //
 // The convolutions carry no bias: with GELU(0) = 0 the network maps a zero
 // residual to a zero correction, so cells where the residual has vanished get
@@ -481,22 +482,22 @@ __global__ void k_pack_wtc_t(const float *__restrict__ wq, Layout L, bf16 *__res
 // weight gradient on the tensor cores.
 __global__ void k_pack_grad16(int64_t n, const float *__restrict__ gout, bf16 *__restrict__ g16)
 {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(gout[i], 0.0f);
-        uint4 *dst = reinterpret_cast<uint4 *>(g16 + i * 16);
-        dst[0] = make_uint4(*reinterpret_cast<const uint32_t *>(&h), 0, 0, 0);
-        dst[1] = make_uint4(0, 0, 0, 0);
+    const int64_t rows = tc::act_rows(n);  // zeros from n on
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(i < n ? gout[i] : 0.0f, 0.0f);
+        tc::put_cell(g16, rows, i, make_uint4(*reinterpret_cast<const uint32_t *>(&h), 0, 0, 0), make_uint4(0, 0, 0, 0));
     }
 }
 
 // Tensor-core input: x16[b][c] = (r s_b, r s_b f, 0 x 14) on interior cells,
-// zeros elsewhere (32 bytes per cell, the layout of the hidden activations).
+// zeros elsewhere (the layout of the hidden activations).
 __global__ void k_pack_input16(GridDiv g, int64_t N, const float *__restrict__ r, const float *__restrict__ feat,
                                const double *__restrict__ rr, double n_int, bf16 *__restrict__ x16,
                                const int *__restrict__ skip)
 {
     if (skip && *((volatile const int *)skip)) return;
     const int b = blockIdx.y;
+    const int64_t cells = N * gridDim.y, rows = tc::act_rows(cells);
     float s = 1.0f;
     if (rr) {
         const double v = rr[b];
@@ -510,10 +511,10 @@ __global__ void k_pack_input16(GridDiv g, int64_t N, const float *__restrict__ r
             const __nv_bfloat162 h = __floats2bfloat162_rn(rs, feat ? rs * feat[o] : 0.0f);
             w0 = *reinterpret_cast<const uint32_t *>(&h);
         }
-        uint4 *dst = reinterpret_cast<uint4 *>(x16 + o * 16);
-        dst[0] = make_uint4(w0, 0, 0, 0);
-        dst[1] = make_uint4(0, 0, 0, 0);
+        tc::put_cell(x16, rows, o, make_uint4(w0, 0, 0, 0), make_uint4(0, 0, 0, 0));
     }
+    const int64_t pad = cells + threadIdx.x;  // the rows after the last cell
+    if (blockIdx.x == 0 && blockIdx.y == 0 && pad < rows) tc::put_cell(x16, rows, pad, make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0));
 }
 
 // Deterministic host RNG for the initial weights (splitmix64 + Box-Muller).
@@ -583,22 +584,22 @@ static int net_reserve(piro_pcnet *n, int64_t cells, bool training)
 {
     if (cells <= n->cap && (!training || n->y[0])) return PIRO_OK;
     net_free_ws(n);
-    const size_t c = (size_t)cells;
+    const size_t c = (size_t)cells, c16 = (size_t)tc::act_rows(cells) * 16;  // and 16 channels in the layout of conv_tc.cuh
     cudaError_t e = cudaMalloc(&n->x0, c * 2 * sizeof(bf16));
-    for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMalloc(&n->a[i], c * 16 * sizeof(bf16));
+    for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMalloc(&n->a[i], c16 * sizeof(bf16));
     if (e == cudaSuccess) e = cudaMalloc(&n->out, c * sizeof(float));
     if (training) {
-        for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMalloc(&n->y[i], c * 16 * sizeof(bf16));
-        for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&n->g16[i], c * 16 * sizeof(bf16));
+        for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMalloc(&n->y[i], c16 * sizeof(bf16));
+        for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&n->g16[i], c16 * sizeof(bf16));
         if (e == cudaSuccess) e = cudaMalloc(&n->gout, c * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&n->x16, c * 16 * sizeof(bf16));
-        if (e == cudaSuccess) e = cudaMalloc(&n->go16, c * 16 * sizeof(bf16));
+        if (e == cudaSuccess) e = cudaMalloc(&n->x16, c16 * sizeof(bf16));
+        if (e == cudaSuccess) e = cudaMalloc(&n->go16, c16 * sizeof(bf16));
         // defined contents before the first pass (every layer writes all of its output)
-        for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMemset(n->y[i], 0, c * 16 * sizeof(bf16));
-        for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMemset(n->g16[i], 0, c * 16 * sizeof(bf16));
+        for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMemset(n->y[i], 0, c16 * sizeof(bf16));
+        for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMemset(n->g16[i], 0, c16 * sizeof(bf16));
         if (e == cudaSuccess) e = cudaMemset(n->out, 0, c * sizeof(float));
     }
-    for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMemset(n->a[i], 0, c * 16 * sizeof(bf16));
+    for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMemset(n->a[i], 0, c16 * sizeof(bf16));
     if (e != cudaSuccess) {
         net_free_ws(n);
         set_error("piro_pcnet: workspace allocation failed: %s", cudaGetErrorString(e));
@@ -662,15 +663,15 @@ static Acts infer_acts(void *work, int64_t cells)
 {
     bf16 *x0 = static_cast<bf16 *>(work);
     bf16 *b0 = x0 + cdiv(cells * 2, 128) * 128;
-    bf16 *b1 = b0 + cells * 16;
+    bf16 *b1 = b0 + tc::act_rows(cells) * 16;
     return Acts{x0, {nullptr, nullptr, nullptr}, {b0, b1, b0}};
 }
 
-// TMA descriptor of an activation array of `rows` cells (16 BF16 channels
-// each) as the 3-D view (8 channels, rows at 32 bytes, 2 groups at 16 bytes)
-// with box {8, box_rows, 2}: the line blocks of conv_tc.cuh (130 rows) or the
-// tiles of wgrad_tc.cuh (128 rows).
-static int encode_rows_map(CUtensorMap *m, const void *base, int64_t rows, int box_rows)
+// TMA descriptor of an activation array of `cells` cells (two planes of 8 BF16
+// channels) as the 4-D view of conv_tc.cuh: (8 rows x 8 channels, first row
+// 0..7, blocks of 8 rows, planes).  The last block read starts in the last
+// whole block and ends in the 8 rows that a plane has beyond those.
+static int encode_rows_map(CUtensorMap *m, const void *base, int64_t cells)
 {
     // the driver entry point, resolved once for all host threads
     static std::once_flag resolved;
@@ -686,11 +687,12 @@ static int encode_rows_map(CUtensorMap *m, const void *base, int64_t rows, int b
         set_error("cuTensorMapEncodeTiled is not available");
         return PIRO_ERR_CUDA;
     }
-    const cuuint64_t dims[3] = {8, (cuuint64_t)rows, 2};
-    const cuuint64_t strides[2] = {32, 16};
-    const cuuint32_t box[3] = {8, (cuuint32_t)box_rows, 2};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(base), dims, strides, box,
+    const int64_t plane = tc::act_rows(cells);
+    const cuuint64_t dims[4] = {64, 8, (cuuint64_t)(plane / 8 - 1), 2};
+    const cuuint64_t strides[3] = {16, 128, (cuuint64_t)plane * 16};
+    const cuuint32_t box[4] = {64, 1, tc::kLineRows / 8, 2};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims, strides, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -719,14 +721,14 @@ static int conv_tc(const bf16 *in, bf16 *out, float *zout, const bf16 *wpk, cons
     });
     if (rc != PIRO_OK) return rc;
     CUtensorMap map;
-    rc = encode_rows_map(&map, in, N * batch, tc::kLineRows);
+    rc = encode_rows_map(&map, in, N * batch);
     if (rc) return rc;
     const int64_t nxy = (int64_t)g.nx * g.ny;
     const int ncol = (int)cdiv(nxy, tc::kRows);
     const int planes = g.nz - 2;
     const int zchunk = planes < kTcZChunk ? planes : kTcZChunk;
     const int nzc = (int)cdiv(planes, zchunk);
-    tc::Args a{g, N, nxy, ncol, zchunk, wpk, out, zout, rr, n_int, skip, err, yout, yprev};
+    tc::Args a{g, N, nxy, ncol, zchunk, wpk, out, zout, rr, n_int, skip, err, N * batch, tc::act_rows(N * batch), yout, yprev};
     tc::k_conv16_tc<kEpi><<<dim3((unsigned)(ncol * nzc), (unsigned)batch), tc::kThreads, tc::kSmemBytes, st>>>(map, a);
     PIRO_CHECK_LAUNCH("k_conv16_tc");
     return PIRO_OK;
@@ -776,8 +778,8 @@ static int launch_wgrad_tc(piro_pcnet *n, const GridDiv &g, int64_t cells, const
     });
     if (rc != PIRO_OK) return rc;
     CUtensorMap xmap, gmap;
-    rc = encode_rows_map(&xmap, x, cells, tc::kWgRows);
-    if (!rc) rc = encode_rows_map(&gmap, gy, cells, tc::kWgRows);
+    rc = encode_rows_map(&xmap, x, cells);
+    if (!rc) rc = encode_rows_map(&gmap, gy, cells);
     if (rc) return rc;
     const int64_t ntiles = cdiv(cells, tc::kWgRows);
     int64_t grid = sm_count();
@@ -930,7 +932,7 @@ extern "C" int piro_pcnet_set_engine(piro_pcnet *n, int engine)
 
 namespace piro {
 // Device bytes of the caller-owned workspace of pcnet_apply for N cells.
-size_t pcnet_apply_bytes(int64_t N) { return sizeof(bf16) * (size_t)(cdiv(N * 2, 128) * 128 + 2 * N * 16); }
+size_t pcnet_apply_bytes(int64_t N) { return sizeof(bf16) * (size_t)(cdiv(N * 2, 128) * 128 + 2 * tc::act_rows(N) * 16); }
 
 // Tensor-core pipeline error of the network (a bounded wait ran out); clears it.
 int pcnet_take_error(const piro_pcnet *n, cudaStream_t st)
