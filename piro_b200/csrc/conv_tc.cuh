@@ -27,18 +27,27 @@
 // fill): before the array and after it there are at least 13 boundary cells,
 // so the part of a block that lies in the array holds zeros too.
 //
-// A CTA owns one 128-cell column and marches it along z: the 9 line blocks of
-// tile z are the 3 of each of the planes z-1, z, z+1, so each new tile loads 3
-// line blocks (one plane) while the others stay resident: a ring of 4 planes
-// (3 in use, 1 loading).  L2 -> SM traffic is about 3 * 136/128 * 32 bytes
-// per output cell, against 27 * 32 for a load per tap.
+// The tiles are numbered along z within a column of 128 cells, the columns of
+// one member after another, and a CTA takes an equal share of that sequence,
+// three CTAs per SM.  Along z the 9 line blocks of tile z are the 3 of each of
+// the planes z-1, z, z+1, so a tile after the first of a column (or of the
+// share) loads 3 line blocks (one plane) while the others stay resident: a ring
+// of 4 planes (3 in use, 1 loading).  L2 -> SM traffic is about 3 * 136/128 * 32
+// bytes per output cell, against 27 * 32 for a load per tap.
 //
-// Batched grids (blockIdx.y = member b) are consecutive in the array: rows
-// b*N .. b*N + N - 1.
+// Bound by operand A's way from shared memory to the tensor pipe, 4 KB per MMA:
+// 32 cycles each, 27 a tile, 48 us of 77 for a 128^3 layer (16128 tiles on 148
+// SMs; B200).  CTAs of 16 tiles each, 2.3 per resident slot, whose MMAs one lane
+// issued from a branch of its own, took 100 us: equal shares of the tiles give 95,
+// and an MMA warp that runs its loops as one, so that the descriptors stay in
+// uniform registers, 77.  Two CTAs per SM with 7 slots and 4 accumulators take
+// 77 as well, one CTA 98, alternating the MMAs of two tiles 92.
+//
+// Batched grids (member b) are consecutive in the array: rows b*N .. b*N + N - 1.
 //
 // Warp roles (192 threads): warps 0-3 read the accumulator (TMEM lanes
 // 32w..32w+31), apply GELU and store; warp 4 lane 0 issues the TMA loads;
-// warp 5 lane 0 issues the MMAs.  Two TMEM accumulators (2 x 16 columns)
+// warp 5 issues the MMAs.  Two TMEM accumulators (2 x 16 columns)
 // overlap a tile's epilogue with the next tile's MMAs (four measured slower).  mbarriers: full[slot]
 // (TMA bytes landed), empty[slot] (the MMAs reading a plane completed),
 // acc_full[b] (a tile's MMAs completed), acc_empty[b] (its epilogue read it).
@@ -67,6 +76,7 @@ constexpr int kBarOff = kSlots * kPlaneBytes + kWBytes;
 constexpr int kAcc = 2;                       // TMEM accumulators (16 columns each) per CTA
 constexpr int kBarSlots = 2 * kSlots + 2 * kAcc + 1;  // full, empty, acc_full, acc_empty, drain
 constexpr int kSmemBytes = kBarOff + kBarSlots * 8 + 16 + 128;  // + barriers, TMEM address, alignment slack
+constexpr int kCtas = 3;                      // per SM
 constexpr long long kSpin = 1ll << 24;        // polls before a wait gives up
 
 // Rows of a plane of an activation array: the stride of its 8-row blocks divides it.
@@ -74,8 +84,8 @@ __host__ __device__ inline int64_t act_rows(int64_t cells) { return (cells + 7) 
 
 struct Args {
     GridDiv g;
-    int64_t N, nxy;
-    int ncol, zchunk;
+    int64_t N, nxy, ntiles;  // ntiles: members x columns x (nz - 2)
+    int ncol;                // columns of 128 cells per member
     const bf16 *wpk;   // packed weights of this layer
     bf16 *out;         // output activations (epilogues 0, 2) or gradient (epilogue 3)
     float *zout;       // FP32 output channel 0 (epilogue 1)
@@ -126,6 +136,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *er
     return false;
 }
 
+// The same for a whole warp.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int *err)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err));
+}
+
 // Wait for a phase that is certain to complete (copies or MMAs this CTA
 // issued itself), with its own bound so that a role which gave up on a
 // partner still leaves nothing in flight behind it.
@@ -165,18 +181,37 @@ __device__ __forceinline__ uint64_t desc_nosw(uint32_t saddr, uint32_t lbo, uint
 // bits 24-28.
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t acc)
+// The MMA warp runs its loops as one and the lane with `issue` set issues: the
+// descriptors stay in uniform registers.  From a branch that one lane takes, an
+// MMA cost its CTA about 100 cycles.
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t acc, uint32_t idesc,
+                                         uint32_t issue)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(acc)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(issue)
         : "memory");
 }
-__device__ __forceinline__ void mma_commit(uint32_t bar)
+__device__ __forceinline__ void mma_commit(uint32_t bar, uint32_t issue)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(issue)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t elect_one()
+{
+    uint32_t e;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(e));
+    return e;
 }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -213,6 +248,44 @@ __device__ __forceinline__ float gelu_d_tc(float x)
     return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 0.134145f * x * x);
 }
 
+// A tile's place: member, column, plane; row: its first cell in the array.
+struct Tile {
+    int64_t b, row;
+    int col, z;
+    __device__ Tile(const Args &a, int64_t t)
+    {
+        const int planes = a.g.nz - 2;
+        const int64_t q = t / planes;
+        z = 1 + (int)(t % planes);
+        b = q / a.ncol;
+        col = (int)(q % a.ncol);
+        row = b * a.N + z * a.nxy + (int64_t)col * kRows;
+    }
+    __device__ void next(const Args &a)
+    {
+        row += a.nxy;
+        if (++z < a.g.nz - 1) return;
+        z = 1;
+        if (++col == a.ncol) {
+            col = 0;
+            ++b;
+        }
+        row = b * a.N + a.nxy + (int64_t)col * kRows;
+    }
+};
+
+template <int kEpi>
+__device__ __forceinline__ void put_zero(const Args &a, int64_t c)
+{
+    const uint4 z4 = make_uint4(0, 0, 0, 0);
+    if (kEpi == 1) {
+        a.zout[c] = 0.0f;
+        return;
+    }
+    put_cell(a.out, a.rows, c, z4, z4);
+    if (kEpi == 2) put_cell(a.yout, a.rows, c, z4, z4);
+}
+
 // kEpi 0: GELU, 16 BF16 channels out (hidden layers); 1: output channel 0 in
 // FP32 times the batch member's scale (the last layer, N padded to 16);
 // 2 (training forward): the pre-activation y = bf16(acc) to yout and GELU(y)
@@ -220,7 +293,7 @@ __device__ __forceinline__ float gelu_d_tc(float x)
 // out = bf16(acc * GELU'(yprev)), the gradient with respect to the previous
 // layer's pre-activation.  Every epilogue writes zeros on non-interior cells.
 template <int kEpi>
-__global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant__ CUtensorMap xmap, Args a)
+__global__ void __launch_bounds__(kThreads, kCtas) k_conv16_tc(const __grid_constant__ CUtensorMap xmap, Args a)
 {
     if (a.skip && *((volatile const int *)a.skip)) return;
     extern __shared__ unsigned char smem_raw[];
@@ -235,12 +308,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
     auto acce = [&](int b) { return bar_s + 8u * (2 * kSlots + kAcc + b); };
     const uint32_t drain_s = bar_s + 8u * (2 * kSlots + 2 * kAcc);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t boff = (int64_t)blockIdx.y * a.N;  // batch member: rows b*N ..
-    const int col = blockIdx.x % a.ncol;
-    const int zb = 1 + (blockIdx.x / a.ncol) * a.zchunk;
-    const int ze = min(zb + a.zchunk, a.g.nz - 1);
-    const int P = ze - zb;  // tiles (output planes) of this CTA
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // uniform, for the compiler
+    const int64_t t0 = a.ntiles * blockIdx.x / gridDim.x;
+    const int P = (int)(a.ntiles * (blockIdx.x + 1) / gridDim.x - t0);  // tiles of this CTA
+    Tile tile(a, t0);
 
     // weights -> shared memory (generic proxy), then made visible to the tensor cores
     {
@@ -270,21 +341,22 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(tmem_slot), 0);
 
     if (P > 0) {
         if (warp == 4) {
             if (lane == 0) {
-                // producer: planes zb-1 .. ze, three line blocks each
-                int p = 0;
-                for (; p < P + 2; ++p) {
-                    const int slot = p % kSlots;
-                    if (p >= kSlots && !mbar_wait(empty(slot), ((p / kSlots) - 1) & 1, a.err)) break;
-                    const int64_t L = zb - 1 + p;
-                    mbar_expect_tx(full(slot), 3 * kLineBytes);
-                    for (int dy = 0; dy < 3; ++dy) {
-                        const int64_t r = boff + L * a.nxy + (int64_t)col * kRows - 1 + (int64_t)(dy - 1) * a.g.nx;
-                        tma_load_rows(planes_s + slot * kPlaneBytes + dy * kLineBytes, &xmap, full(slot), r);
+                // producer: a tile's new planes, three line blocks each
+                int p = 0;  // planes loaded
+                bool ok = true;
+                for (int j = 0; j < P && ok; ++j, tile.next(a)) {
+                    for (int k = j == 0 || tile.z == 1 ? 0 : 2; k < 3; ++k, ++p) {
+                        const int slot = p % kSlots;
+                        if (p >= kSlots && !(ok = mbar_wait(empty(slot), ((p / kSlots) - 1) & 1, a.err))) break;
+                        mbar_expect_tx(full(slot), 3 * kLineBytes);
+                        for (int dy = 0; dy < 3; ++dy)
+                            tma_load_rows(planes_s + slot * kPlaneBytes + dy * kLineBytes, &xmap, full(slot),
+                                          tile.row + (int64_t)(k - 1) * a.nxy - 1 + (int64_t)(dy - 1) * a.g.nx);
                     }
                 }
                 // no copy may land after the CTA has left, whatever the other
@@ -292,63 +364,49 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                 for (int q = p - kSlots < 0 ? 0 : p - kSlots; q < p; ++q) mbar_drain(full(q % kSlots), (q / kSlots) & 1);
             }
         } else if (warp == 5) {
-            if (lane == 0) {
-                int waited = 0;
+            {
+                const uint32_t issue = elect_one();
+                // a move of the start address is an addition to the descriptor's low bits
+                const uint64_t a0 = desc_nosw(planes_s, kLineRows * 16, 128), b0 = desc_nosw(w_s, 256, 128);
+                int waited = 0, p = 0;  // p: the tile's first plane, in the order of loading
                 bool ok = true;
                 for (int j = 0; j < P && ok; ++j) {
-                    while (ok && waited < j + 3) {
-                        ok = mbar_wait(full(waited % kSlots), (waited / kSlots) & 1, a.err);
+                    while (ok && waited < p + 3) {
+                        ok = mbar_wait_warp(full(waited % kSlots), (waited / kSlots) & 1, a.err);
                         ++waited;
                     }
                     const int buf = j % kAcc;
-                    if (ok && j >= kAcc) ok = mbar_wait(acce(buf), ((j / kAcc) - 1) & 1, a.err);
+                    if (ok && j >= kAcc) ok = mbar_wait_warp(acce(buf), ((j / kAcc) - 1) & 1, a.err);
                     if (!ok) break;
                     fence_after();
                     const uint32_t d_tmem = tmem + (uint32_t)(buf * 16);
-#pragma unroll 1
+#pragma unroll
                     for (int dz = 0; dz < 3; ++dz) {
-                        const uint32_t pbase = planes_s + ((j + dz) % kSlots) * kPlaneBytes;
+                        const uint64_t ab = a0 + (uint32_t)((p + dz) % kSlots) * (kPlaneBytes / 16);
 #pragma unroll
                         for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
                             for (int dx = 0; dx < 3; ++dx) {
                                 const int tap = dz * 9 + dy * 3 + dx;
-                                const uint64_t ad =
-                                    desc_nosw(pbase + dy * kLineBytes + dx * 16, kLineRows * 16, 128);
-                                const uint64_t bd = desc_nosw(w_s + tap * 512, 256, 128);
-                                mma_bf16(d_tmem, ad, bd, tap > 0 ? 1u : 0u);
+                                mma_bf16(d_tmem, ab + (dy * kLineBytes / 16 + dx), b0 + tap * 32, tap > 0 ? 1u : 0u, kIdesc, issue);
                             }
                     }
-                    mma_commit(accf(buf));
-                    mma_commit(empty(j % kSlots));  // plane z-1 is read by no later tile
+                    mma_commit(accf(buf), issue);
+                    // plane z-1 is read by no later tile; at the end of a column no plane is
+                    tile.next(a);
+                    mma_commit(empty(p++ % kSlots), issue);
+                    if (tile.z == 1) {
+                        mma_commit(empty(p++ % kSlots), issue);
+                        mma_commit(empty(p++ % kSlots), issue);
+                    }
                 }
                 // every MMA issued here has completed before TMEM is released
-                mma_commit(drain_s);
+                mma_commit(drain_s, issue);
                 mbar_drain(drain_s, 0);
             }
         } else {
-            // the boundary planes z = 0 and nz - 1 of this column hold zeros
-            // in every output (no tile computes them; a buffer reused for
-            // another grid must not keep values there)
-            for (int e = 0; e < 2; ++e) {
-                if ((e == 0 && zb != 1) || (e == 1 && ze != a.g.nz - 1)) continue;
-                const int64_t inplane = (int64_t)col * kRows + warp * 32 + lane;
-                if (inplane >= a.nxy) continue;
-                const int64_t c = (e == 0 ? 0 : (int64_t)(a.g.nz - 1) * a.nxy) + inplane;
-                if (kEpi == 1) {
-                    a.zout[boff + c] = 0.0f;
-                } else {
-                    const uint4 z4 = make_uint4(0, 0, 0, 0);
-                    put_cell(a.out, a.rows, boff + c, z4, z4);
-                    if (kEpi == 2) put_cell(a.yout, a.rows, boff + c, z4, z4);
-                }
-            }
-            // and so do the rows after the last cell (the next layer's loads read them)
-            if (kEpi != 1 && warp == 0 && boff + a.N == a.cells && ze == a.g.nz - 1 && col == a.ncol - 1 &&
-                a.cells + lane < a.rows)
-                put_cell(a.out, a.rows, a.cells + lane, make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0));
             // epilogue: warp w holds tile rows 32w .. 32w+31
-            for (int j = 0; j < P; ++j) {
+            for (int j = 0; j < P; ++j, tile.next(a)) {
                 const int buf = j % kAcc;
                 if (!mbar_wait(accf(buf), (j / kAcc) & 1, a.err)) break;
                 fence_after();
@@ -357,11 +415,22 @@ __global__ void __launch_bounds__(kThreads, 3) k_conv16_tc(const __grid_constant
                 fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acce(buf));
-                const int64_t c = (int64_t)(zb + j) * a.nxy + (int64_t)col * kRows + warp * 32 + lane;
+                const int64_t inplane = (int64_t)tile.col * kRows + warp * 32 + lane, boff = tile.b * a.N;
+                const int64_t c = (int64_t)tile.z * a.nxy + inplane;
+                // the boundary planes z = 0 and nz - 1 of a column hold zeros in every
+                // output (no tile computes them; a buffer reused for another grid must
+                // not keep values there), and so do the rows after the last cell (the
+                // next layer's loads read them)
+                if (inplane < a.nxy) {
+                    if (tile.z == 1) put_zero<kEpi>(a, boff + inplane);
+                    if (tile.z == a.g.nz - 2) put_zero<kEpi>(a, boff + c + a.nxy);
+                }
+                if (kEpi != 1 && t0 + j == a.ntiles - 1 && warp == 0 && a.cells + lane < a.rows)
+                    put_cell(a.out, a.rows, a.cells + lane, make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0));
                 if (kEpi == 1) {
                     if (c < a.N) {
                         float sc = 1.0f;
-                        if (a.rr) sc = (float)sqrt(a.rr[blockIdx.y] / a.n_int);
+                        if (a.rr) sc = (float)sqrt(a.rr[tile.b] / a.n_int);
                         a.zout[boff + c] = a.g.interior(c) ? __uint_as_float(v[0]) * sc : 0.0f;
                     }
                 } else if (kEpi == 3) {

@@ -49,7 +49,6 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int kTaps = 27;
 constexpr int kLayers = 4;
-constexpr int kTcZChunk = 16;  // z-planes per CTA of the tensor-core layers
 constexpr int kCi[kLayers] = {2, 16, 16, 16};
 constexpr int kCo[kLayers] = {16, 16, 16, 1};
 
@@ -725,11 +724,10 @@ static int conv_tc(const bf16 *in, bf16 *out, float *zout, const bf16 *wpk, cons
     if (rc) return rc;
     const int64_t nxy = (int64_t)g.nx * g.ny;
     const int ncol = (int)cdiv(nxy, tc::kRows);
-    const int planes = g.nz - 2;
-    const int zchunk = planes < kTcZChunk ? planes : kTcZChunk;
-    const int nzc = (int)cdiv(planes, zchunk);
-    tc::Args a{g, N, nxy, ncol, zchunk, wpk, out, zout, rr, n_int, skip, err, N * batch, tc::act_rows(N * batch), yout, yprev};
-    tc::k_conv16_tc<kEpi><<<dim3((unsigned)(ncol * nzc), (unsigned)batch), tc::kThreads, tc::kSmemBytes, st>>>(map, a);
+    const int64_t ntiles = (int64_t)batch * ncol * (g.nz - 2);
+    const int64_t grid = ntiles < tc::kCtas * sm_count() ? ntiles : tc::kCtas * sm_count();
+    tc::Args a{g, N, nxy, ntiles, ncol, wpk, out, zout, rr, n_int, skip, err, N * batch, tc::act_rows(N * batch), yout, yprev};
+    tc::k_conv16_tc<kEpi><<<(unsigned)grid, tc::kThreads, tc::kSmemBytes, st>>>(map, a);
     PIRO_CHECK_LAUNCH("k_conv16_tc");
     return PIRO_OK;
 }

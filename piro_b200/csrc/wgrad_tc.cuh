@@ -33,8 +33,8 @@
 // meets only G = 0 there (G vanishes off the interior, and an interior cell's
 // 27 neighbours lie inside its own member).
 //
-// Warp roles (192 threads): warp 4 lane 0 issues the TMA loads, warp 5 lane 0
-// the MMAs, warps 0-3 read the accumulators out at the end (TMEM lanes
+// Warp roles (192 threads): warp 4 lane 0 issues the TMA loads, warp 5 the
+// MMAs, warps 0-3 read the accumulators out at the end (TMEM lanes
 // 32w..32w+31).  mbarriers: full[s] (a stage's 12 blocks landed), empty[s] (the
 // MMAs reading the stage completed), done (every MMA completed).  Every wait
 // is bounded; a role that gives up raises *err, and the producer and the MMA
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_tc(const __grid_constan
     const uint32_t done_s = bar_s + 8u * (2 * kWgStages);
     const uint32_t drain_s = bar_s + 8u * (2 * kWgStages + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // uniform, for the compiler
     const int64_t my_tiles = (int64_t)blockIdx.x < a.ntiles ? (a.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
     if (threadIdx.x == 0) {
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_tc(const __grid_constan
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(tmem_slot), 0);
     bool mma_ok = my_tiles > 0;
 
     if (warp == 4) {
@@ -126,34 +126,25 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_tc(const __grid_constan
                 mbar_drain(full((int)(q % kWgStages)), (uint32_t)((q / kWgStages) & 1));
         }
     } else if (warp == 5) {
-        if (lane == 0 && my_tiles > 0) {
+        if (my_tiles > 0) {
+            const uint32_t issue = elect_one();
+            const uint64_t x0 = desc_nosw(stage_s, 128, kLineBytes / 2);  // a move of the start address adds to the low bits
             for (int64_t i = 0; i < my_tiles && mma_ok; ++i) {
                 const int s = (int)(i % kWgStages);
-                if (!(mma_ok = mbar_wait(full(s), (uint32_t)((i / kWgStages) & 1), a.err))) break;
+                if (!(mma_ok = mbar_wait_warp(full(s), (uint32_t)((i / kWgStages) & 1), a.err))) break;
                 fence_after();
-                const uint32_t st = stage_s + (uint32_t)s * kWgStageBytes;
+                const uint64_t st = x0 + (uint32_t)s * (kWgStageBytes / 16);
 #pragma unroll
-                for (int d = 0; d < kWgAcc; ++d) {
-                    const uint32_t d_tmem = tmem + (uint32_t)(d * 16);
-                    const uint32_t as = d < 3 ? st + kWgX + d * 16 : st;
+                for (int d = 0; d < kWgAcc; ++d)
 #pragma unroll
-                    for (int ks = 0; ks < kWgRows / 16; ++ks) {
-                        const uint64_t ad = desc_nosw(as + ks * 256, 128, kLineBytes / 2);
-                        const uint64_t bd = desc_nosw(st + kWgG + ks * 256, 128, kLineBytes / 2);
-                        const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\t"
-                            "setp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                            "l"(ad), "l"(bd), "r"(kIdescMN), "r"(acc)
-                            : "memory");
-                    }
-                }
-                mma_commit(empty(s));
+                    for (int ks = 0; ks < kWgRows / 16; ++ks)
+                        mma_bf16(tmem + (uint32_t)(d * 16), st + ((d < 3 ? kWgX / 16 + d : 0) + ks * 16), st + (kWgG / 16 + ks * 16),
+                                 (i > 0 || ks > 0) ? 1u : 0u, kIdescMN, issue);
+                mma_commit(empty(s), issue);
             }
-            mma_commit(done_s);
+            mma_commit(done_s, issue);
             // every MMA issued here has completed before TMEM is read or released
-            mma_commit(drain_s);
+            mma_commit(drain_s, issue);
             mbar_drain(drain_s, 0);
         }
     } else {

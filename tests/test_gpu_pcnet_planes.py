@@ -42,3 +42,22 @@ def test_planes_do_not_depend_on_what_was_there(cuda, n, B):
     for l in range(4):  # BF16 activations and gradients: 2^-8 per rounding, a few roundings deep
         a, b = got[0][1][wo[l]:ends[l]].astype(np.float64), rg[wo[l]:ends[l]]
         assert np.sqrt(((a - b) ** 2).sum()) <= 2e-2 * np.sqrt((b ** 2).sum()), l
+
+
+@pytest.mark.parametrize("n,B", [((33, 31, 6), 40), ((34, 34, 9), 12), ((6, 5, 3), 700), ((12, 12, 400), 3)])
+def test_shares_of_the_tiles_do_not_matter(cuda, n, B):
+    """A batch and its members alone, whose tiles fall to other blocks (one tile
+    a block, shares that end inside a column, at its end and in the next
+    member): the same bits."""
+    import torch
+    from piro_b200 import ops
+    rng = np.random.default_rng(4)
+    N = n[0] * n[1] * n[2]
+    r, f = (torch.from_numpy(rng.standard_normal(B * N).astype(np.float32)).cuda() for _ in range(2))
+    net = ops.PCNet(seed=0)
+    out = net.forward(*n, r, f, batch=B)
+    for b in sorted({0, 1, B // 2, B - 2, B - 1}):
+        s = slice(b * N, (b + 1) * N)
+        one = net.forward(*n, r[s].contiguous(), f[s].contiguous())
+        assert torch.equal(out[s].view(torch.int32), one.view(torch.int32)), b
+    net.close()
