@@ -356,12 +356,20 @@ __global__ void __launch_bounds__(256) k_conv_bwd_w(GridDiv g, int64_t N, int B,
     }
 }
 
-// out[p] = sum over blocks (fixed order, FP64) of partials[block][p].
-__global__ void k_reduce_partials(const float *__restrict__ partials, int nblocks, int P, float *__restrict__ out)
+// out[p] = sum over blocks (fixed order, FP64) of partials[block][p].  Bound by
+// the latency of the loads, 32 of them at a time: 148 partials of 6912 values take
+// 17 us, four at a time they took 22 (B200).
+__global__ void __launch_bounds__(64) k_reduce_partials(const float *__restrict__ partials, int nblocks, int P, float *__restrict__ out)
 {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
         double s = 0.0;
-        for (int k = 0; k < nblocks; ++k) s += (double)partials[(int64_t)k * P + p];
+        for (int k0 = 0; k0 < nblocks; k0 += 32) {
+            float v[32];
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = partials[(int64_t)(k0 + k < nblocks ? k0 + k : nblocks - 1) * P + p];
+#pragma unroll
+            for (int k = 0; k < 32; ++k) s += k0 + k < nblocks ? (double)v[k] : 0.0;  // + 0: s is never -0
+        }
         out[p] = (float)s;
     }
 }
@@ -385,12 +393,18 @@ __global__ void __launch_bounds__(256) k_mask_sum(int64_t n, const float *__rest
     }
 }
 
-// Sum the kRedBlocks partials in order into red[kRedBlocks + slot].
+// Sum the kRedBlocks partials in order into red[kRedBlocks + slot] (one block of
+// at least kRedBlocks threads).  Bound by the serial sum, 4 us; with the loads in it
+// as well 13 (B200).
 __global__ void k_finish_sum(double *red, int slot)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
+    __shared__ double s_red[kRedBlocks];
+    if (threadIdx.x < kRedBlocks) s_red[threadIdx.x] = red[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
         double s = 0.0;
-        for (int k = 0; k < kRedBlocks; ++k) s += red[k];
+#pragma unroll 8
+        for (int k = 0; k < kRedBlocks; ++k) s += s_red[k];
         red[kRedBlocks + slot] = s;
     }
 }
@@ -787,7 +801,7 @@ static int launch_wgrad_tc(piro_pcnet *n, const GridDiv &g, int64_t cells, const
     tc::k_wgrad_tc<<<(unsigned)grid, tc::kWgThreads, tc::kWgSmemBytes, st>>>(xmap, gmap, a);
     PIRO_CHECK_LAUNCH("k_wgrad_tc");
     const int P = kTaps * CI * CO;
-    k_reduce_partials<<<(P + 255) / 256, 256, 0, st>>>(n->partials, (int)grid, P, grad_w);
+    k_reduce_partials<<<(P + 63) / 64, 64, 0, st>>>(n->partials, (int)grid, P, grad_w);
     PIRO_CHECK_LAUNCH("k_reduce_partials");
     n->launches += 2;
     return PIRO_OK;
@@ -810,7 +824,7 @@ static int launch_bwd_w(piro_pcnet *n, const GridDiv &g, int64_t N, int batch, c
     const int nblocks = kRedBlocks;
     constexpr int P = kTaps * CI * CO;
     k_conv_bwd_w<CI, CO, GT><<<nblocks, 256, smem, st>>>(g, N, batch, x, gy, n->partials);
-    k_reduce_partials<<<(P + 255) / 256, 256, 0, st>>>(n->partials, nblocks, P, grad_w);
+    k_reduce_partials<<<(P + 63) / 64, 64, 0, st>>>(n->partials, nblocks, P, grad_w);
     n->launches += 2;
     PIRO_CHECK_LAUNCH("k_conv_bwd_w");
     return PIRO_OK;
@@ -999,9 +1013,9 @@ extern "C" int piro_pcnet_loss_grad(piro_pcnet *n, int batch, int nx, int ny, in
     n->launches += 5;
     if (rc) return rc;
     k_mask_sum<<<kRedBlocks, 256, 0, st>>>(cells, mask, n->red);
-    k_finish_sum<<<1, 32, 0, st>>>(n->red, 0);
+    k_finish_sum<<<1, 320, 0, st>>>(n->red, 0);
     k_loss<<<kRedBlocks, 256, 0, st>>>(g, N, cells, n->out, target, mask, n->red, n->gout);
-    k_finish_sum<<<1, 32, 0, st>>>(n->red, 1);
+    k_finish_sum<<<1, 320, 0, st>>>(n->red, 1);
     PIRO_CHECK_LAUNCH("k_loss");
     const dim3 grid(net_grid(N, 128), batch);
     if (tcore) {

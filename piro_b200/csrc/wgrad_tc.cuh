@@ -23,7 +23,7 @@
 // never used).  With operand B's (N = 16) that is 12 blocks a tile in 408 pieces
 // of 128 bytes.  A block per tap and operand from channels-last cells, 36 a tile
 // in 9216 pieces of 16 bytes, took 210 us for 16 crops of 34^3, bound by the
-// pieces (12 thousand cycles a tile); now 48 (B200).  One MMA covers K = 16 cells
+// pieces (12 thousand cycles a tile); now 34 (B200).  One MMA covers K = 16 cells
 // (descriptor start + 256 bytes per step), 8 steps a tile of 128 cells.  Each of
 // the four MMAs accumulates into its own 16 TMEM columns over every tile the
 // CTA takes; at the end the four accumulators are the CTA's partial dW.
