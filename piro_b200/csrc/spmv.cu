@@ -492,15 +492,27 @@ __global__ void k_scale_add(int64_t n, float dt, const float *acc, const float *
 }
 
 // HT lookup with linear probing (SpMVHT.cl:1-20) from slot h on; bounded by
-// ts probes.
-__device__ __forceinline__ float ht_get_from(int64_t key, int64_t h, const int64_t *__restrict__ keys,
-                                             const float *__restrict__ vals, int64_t ts)
+// the table's length.  Four slots at a time: a warp walks as far as its longest
+// chain, and a slot by itself costs a load's latency.  With the staged step at
+// 256^3 (1178 us; 64^3 35): one slot at a time 1294 (54), three 1162 (38), eight
+// 1248 (37) (B200).
+template <typename I>
+__device__ __forceinline__ float ht_get_from(int64_t key, I h, const int64_t *__restrict__ keys,
+                                             const float *__restrict__ vals, I ts)
 {
-    for (int64_t a = 0; a < ts; ++a) {
-        const int64_t k = __ldg(keys + h);
-        if (k == key) return __ldg(vals + h);
-        if (k == -1) return 0.0f;
-        h = h + 1 == ts ? 0 : h + 1;
+    for (I a = 0; a < ts; a += 4) {
+        I s[4];
+        int64_t k[4];
+        s[0] = h;
+#pragma unroll
+        for (int q = 1; q < 4; ++q) s[q] = s[q - 1] + 1 == ts ? 0 : s[q - 1] + 1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) k[q] = __ldg(keys + s[q]);
+        I at = -2;  // where the walk ends: the first slot with the key, or -1 at an empty one
+#pragma unroll
+        for (int q = 3; q >= 0; --q) at = k[q] == key ? s[q] : k[q] == -1 ? (I)-1 : at;
+        if (at != -2) return at < 0 ? 0.0f : __ldg(vals + at);
+        h = s[3] + 1 == ts ? 0 : s[3] + 1;
     }
     return 0.0f;
 }
@@ -573,12 +585,15 @@ __global__ void __launch_bounds__(256, 4) k_ht_spmv(GridDiv g, int64_t N, const 
 // stores: whole sectors, no read-modify-write of a partly written sector).
 // Pass 2 (rows in index order) reads the records and u coalesced and writes
 // out coalesced.  The per-row arithmetic is the one above, term for term.
-__global__ void __launch_bounds__(256, 4) k_ht_stage(GridDiv g, int64_t N, const int64_t *__restrict__ keys,
-                           const float *__restrict__ vals, int64_t ts, ModU64 mts, const int32_t *__restrict__ order,
-                           float4 *__restrict__ stage)
+// I: the type of a slot, 32 bits where base + off cannot overflow.  Five blocks per
+// SM: four take 1199 us at 256^3, six 1282.
+template <typename I>
+__global__ void __launch_bounds__(256, 5) k_ht_stage(GridDiv g, int64_t N, const int64_t *__restrict__ keys,
+                                                     const float *__restrict__ vals, I ts, ModU64 mts,
+                                                     const int32_t *__restrict__ order, float4 *__restrict__ stage)
 {
     const int nx = g.nx, ny = g.ny, nz = g.nz;
-    const int64_t sxy = (int64_t)nx * ny;
+    const I sxy = (I)nx * (I)ny;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int32_t next_i = j < N ? __ldg(order + j) : 0;  // the row of the next iteration, loaded one ahead
@@ -587,11 +602,12 @@ __global__ void __launch_bounds__(256, 4) k_ht_stage(GridDiv g, int64_t N, const
         if (j + stride < N) next_i = __ldg(order + j + stride);
         int x, y, z;
         g.coords((uint32_t)i, x, y, z);
-        const int64_t off[7] = {-sxy, -(int64_t)nx, -1, 0, 1, (int64_t)nx, sxy};
+        const I off[7] = {-sxy, -(I)nx, -1, 0, 1, (I)nx, sxy};
         const bool ok[7] = {z > 0, y > 0, x > 0, true, x < nx - 1, y < ny - 1, z < nz - 1};
-        const int64_t kd = i * N + i, base = (int64_t)mts.mod((uint64_t)kd);
+        const int64_t kd = i * N + i;
+        const I base = (I)mts.mod((uint64_t)kd);
         auto home = [&](int t) {  // the first probe of candidate t (recomputed on a collision, not kept)
-            int64_t hh = base + off[t];
+            I hh = base + off[t];
             hh += hh < 0 ? ts : 0;
             hh -= hh >= ts ? ts : 0;
             return hh;
@@ -603,7 +619,7 @@ __global__ void __launch_bounds__(256, 4) k_ht_stage(GridDiv g, int64_t N, const
         for (int t = 0; t < 7; ++t) {
             v[t] = 0.0f;
             if (ok[t]) {
-                const int64_t hh = home(t);
+                const I hh = home(t);
                 k[t] = __ldg(keys + hh);
                 v[t] = __ldg(vals + hh);  // with the key: one round trip
             }
@@ -616,8 +632,8 @@ __global__ void __launch_bounds__(256, 4) k_ht_stage(GridDiv g, int64_t N, const
                 } else if (k[t] == -1) {
                     v[t] = 0.0f;
                 } else {
-                    const int64_t hh = home(t);
-                    v[t] = ht_get_from(key, hh + 1 == ts ? 0 : hh + 1, keys, vals, ts);
+                    const I hh = home(t);
+                    v[t] = ht_get_from<I>(key, hh + 1 == ts ? 0 : hh + 1, keys, vals, ts);
                 }
             }
         }
@@ -1458,7 +1474,10 @@ extern "C" int piro_ht_spmv_staged(int nx, int ny, int nz, const int64_t *keys, 
     cudaStream_t s = as_stream(stream);
     float4 *st = static_cast<float4 *>(stage);
     const GridDiv g(nx, ny, nz);
-    k_ht_stage<<<grid_for(N, 256, 8), 256, 0, s>>>(g, N, keys, vals, ts, ModU64((uint64_t)ts), order, st);
+    if (ts < (1 << 30))
+        k_ht_stage<int32_t><<<grid_for(N, 256, 8), 256, 0, s>>>(g, N, keys, vals, (int32_t)ts, ModU64((uint64_t)ts), order, st);
+    else
+        k_ht_stage<int64_t><<<grid_for(N, 256, 8), 256, 0, s>>>(g, N, keys, vals, ts, ModU64((uint64_t)ts), order, st);
     PIRO_CHECK_LAUNCH("k_ht_stage");
     k_ht_stage_apply<<<grid_for(N, 256, 8), 256, 0, s>>>(g, dt, fe, st, u, out);
     PIRO_CHECK_LAUNCH("k_ht_stage_apply");
