@@ -45,6 +45,10 @@ constexpr int kChunkF = 4;      // flexible-CG (Jacobi) iterations per graph lau
 // iterations a second one saves.
 constexpr int kLearnedIters = 1;
 constexpr int kRedCap = 4096;   // max blocks of a reducing kernel
+// Blocks of a reducing kernel: as many as are resident.  With up to kRedCap each
+// wave of blocks publishes, and the last block gathers, that many more partials
+// (128^3, B200: k_residual_mf 50 us against 35, k_fcg_spmv_mf 44 against 29).
+inline int64_t mf_blocks() { return std::min<int64_t>(kRedCap, 8 * sm_count()); }
 
 struct DevState {
     double rz;      // <s, z> of the current iterate
@@ -83,6 +87,24 @@ __device__ __forceinline__ double block_sum(double v, double *s_warp)
     return t;  // thread 0
 }
 
+// kN sums at once (thread 0's tot); s_warp: kN x 32.
+template <int kN>
+__device__ __forceinline__ void block_sums(const double (&v)[kN], double (&tot)[kN], double *s_warp)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kN; ++t) {
+        const double x = warp_sum(v[t]);
+        if (lane == 0) s_warp[t * 32 + w] = x;
+    }
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+        for (int t = 0; t < kN; ++t) tot[t] = warp_sum(lane < (int)(blockDim.x >> 5) ? s_warp[t * 32 + lane] : 0.0);
+    }
+}
+
 // Publish one partial per block; returns true in the block that arrives last
 // (all partials of the launch are then visible to it).
 __device__ __forceinline__ bool publish_last(double *partials, int slot_stride, int nvals, const double *vals,
@@ -99,10 +121,24 @@ __device__ __forceinline__ bool publish_last(double *partials, int slot_stride, 
     return *s_last;
 }
 
+// The partials of kN sums, as gather_sum's, a block barrier pair for all.
+template <int kN>
+__device__ __forceinline__ void gather_sums(const double *partials, double (&tot)[kN], double *s_warp)
+{
+    double s[kN];
+#pragma unroll
+    for (int t = 0; t < kN; ++t) s[t] = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
+#pragma unroll
+        for (int t = 0; t < kN; ++t) s[t] += __ldcg(partials + t * kRedCap + k);
+    }
+    block_sums<kN>(s, tot, s_warp);
+}
+
 __device__ __forceinline__ double gather_sum(const double *partials, double *s_warp)
 {
     double s = 0.0;
-    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) s += ((volatile const double *)partials)[k];
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) s += __ldcg(partials + k);
     return block_sum(s, s_warp);
 }
 
@@ -152,7 +188,7 @@ __global__ void __launch_bounds__(kRowThreads) k_residual(GridDiv g, int64_t N,
                                                         float *__restrict__ z, double *__restrict__ partials,
                                                         DevState *__restrict__ st, double rtol, double inner_floor)
 {
-    __shared__ double s_warp[32];
+    __shared__ double s_warp[4 * 32];
     __shared__ bool s_last;
     ResidualRow op{g, alpha, dinv, b, x, r, z, 0.0, 0.0, 0.0, 0.0, 0.0};
     csr_for_rows(N, rowptr, col, val, op);
@@ -165,11 +201,11 @@ __device__ __forceinline__ void residual_finish(double rr64, double bb, double r
                                                 double *__restrict__ partials, DevState *__restrict__ st, double rtol,
                                                 double inner_floor, double *s_warp, bool *s_last)
 {
-    double part[4] = {block_sum(rr64, s_warp), block_sum(bb, s_warp), block_sum(rz, s_warp),
-                      block_sum(rr32, s_warp)};
+    const double mine[4] = {rr64, bb, rz, rr32};
+    double part[4], tot[4];
+    block_sums<4>(mine, part, s_warp);
     if (!publish_last(partials, kRedCap, 4, part, &st->ticket[0], s_last)) return;
-    double tot[4];
-    for (int t = 0; t < 4; ++t) tot[t] = gather_sum(partials + t * kRedCap, s_warp);
+    gather_sums<4>(partials, tot, s_warp);
     if (threadIdx.x == 0) {
         const double bn = sqrt(tot[1]) > 0.0 ? sqrt(tot[1]) : 1.0;
         const double rel = sqrt(tot[0]) / bn;
@@ -198,7 +234,9 @@ __device__ __forceinline__ void residual_finish(double rr64, double bb, double r
 // entries taken exactly from A (ib_*, PIRO's 10.0 values included), with x
 // holding b on the boundary: the same r = b - A x in FP64 as k_residual
 // (the terms summed in another order), without streaming A's 8 bytes per
-// nonzero.
+// nonzero.  Bound by latency: at 128^3 30 us (67 MB, 10 us of bandwidth), 50 with
+// four times the blocks, four sums gathered one after another and the boundary
+// neighbours' loads in conditions (B200).
 __global__ void __launch_bounds__(256) k_residual_mf(GridDiv g, int64_t N, float mdt, float vself, float vnb,
                                                      const int32_t *__restrict__ ib_ptr,
                                                      const int32_t *__restrict__ ib_col,
@@ -208,7 +246,7 @@ __global__ void __launch_bounds__(256) k_residual_mf(GridDiv g, int64_t N, float
                                                      float *__restrict__ z, double *__restrict__ partials,
                                                      DevState *__restrict__ st, double rtol, double inner_floor)
 {
-    __shared__ double s_warp[32];
+    __shared__ double s_warp[4 * 32];
     __shared__ bool s_last;
     double rr64 = 0.0, bb = 0.0, rz = 0.0, rr32 = 0.0;
     const int64_t sxy = (int64_t)g.nx * g.ny;
@@ -223,15 +261,18 @@ __global__ void __launch_bounds__(256) k_residual_mf(GridDiv g, int64_t N, float
         const float a = __ldg(alpha + i);
         const double cd = (double)__fadd_rn(1.0f, __fmul_rn(mdt, __fmul_rn(a, vself)));
         const double co = (double)__fmul_rn(mdt, __fmul_rn(a, vnb));
-        const double nb = ((xc > 1 ? x[i - 1] : 0.0) + (xc < g.nx - 2 ? x[i + 1] : 0.0)) +
-                          ((y > 1 ? x[i - g.nx] : 0.0) + (y < g.ny - 2 ? x[i + g.nx] : 0.0)) +
-                          ((zc > 1 ? x[i - sxy] : 0.0) + (zc < g.nz - 2 ? x[i + sxy] : 0.0));
-        double q = cd * x[i] + co * nb;
-        for (int32_t k = ib_ptr[i]; k < ib_ptr[i + 1]; ++k) q += (double)ib_val[k] * x[ib_col[k]];
-        const double bi = (double)b[i];
+        // every load before the first use: a load in a condition waits for its own
+        const double xl = __ldg(x + i - 1), xr = __ldg(x + i + 1), yl = __ldg(x + i - g.nx), yr = __ldg(x + i + g.nx);
+        const double zl = __ldg(x + i - sxy), zr = __ldg(x + i + sxy), xi = __ldg(x + i), bi = (double)__ldg(b + i);
+        const float di = __ldg(dinv + i);
+        const int32_t k0 = __ldg(ib_ptr + i), k1 = __ldg(ib_ptr + i + 1);
+        const double nb = ((xc > 1 ? xl : 0.0) + (xc < g.nx - 2 ? xr : 0.0)) + ((y > 1 ? yl : 0.0) + (y < g.ny - 2 ? yr : 0.0)) +
+                          ((zc > 1 ? zl : 0.0) + (zc < g.nz - 2 ? zr : 0.0));
+        double q = cd * xi + co * nb;
+        for (int32_t k = k0; k < k1; ++k) q += (double)ib_val[k] * x[ib_col[k]];
         const double ri = bi - q;
         const float rf = (float)ri;
-        const float zf = rf * dinv[i];
+        const float zf = rf * di;
         r[i] = rf;
         z[i] = zf;
         rr64 += ri * ri;
@@ -575,7 +616,7 @@ __global__ void __launch_bounds__(kMfThreads) k_fcg_spmv_mf(GridDiv g, int64_t N
                                                              float *__restrict__ q, double *__restrict__ partials,
                                                              DevState *__restrict__ st)
 {
-    __shared__ double s_warp[32];
+    __shared__ double s_warp[2 * 32];
     __shared__ bool s_last;
     __shared__ int s_done;
     __shared__ float s_beta;
@@ -612,10 +653,11 @@ __global__ void __launch_bounds__(kMfThreads) k_fcg_spmv_mf(GridDiv g, int64_t N
             q[i] = 0.0f;
         }
     }
-    double part[2] = {block_sum(pq, s_warp), block_sum(pr, s_warp)};
+    const double mine[2] = {pq, pr};
+    double part[2], tot[2];
+    block_sums<2>(mine, part, s_warp);
     if (!publish_last(partials, kRedCap, 2, part, &st->ticket[1], &s_last)) return;
-    double tot[2];
-    for (int t = 0; t < 2; ++t) tot[t] = gather_sum(partials + t * kRedCap, s_warp);
+    gather_sums<2>(partials, tot, s_warp);
     if (threadIdx.x == 0) {
         const double aa = tot[1] / tot[0];
         st->pq = tot[0];
@@ -648,9 +690,10 @@ __global__ void __launch_bounds__(256) k_fcg_update(int64_t N, const float *__re
     const float a = s_a;
     double rr = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        if (dinv[i] == 0.0f) continue;
-        d[i] += a * p[i];
-        const float ri = r[i] - a * q[i];
+        const float di = __ldg(dinv + i), pi = __ldg(p + i), qi = __ldg(q + i), dd = d[i], ro = r[i];
+        if (di == 0.0f) continue;
+        d[i] = dd + a * pi;
+        const float ri = ro - a * qi;
         r[i] = ri;
         rr += (double)ri * (double)ri;
     }
@@ -1877,7 +1920,7 @@ static int be_create(int nx, int ny, int nz, const int32_t *rowptr, const int32_
     }
     const int64_t N = s->N;
     s->grid_tiles = csr_rows_grid(N);
-    s->grid_elem = (unsigned)std::min<int64_t>(std::max<int64_t>(1, cdiv(N / 4, 256)), (int64_t)kRedCap);
+    s->grid_elem = (unsigned)std::min<int64_t>(std::max<int64_t>(1, cdiv(N / 4, 256)), mf_blocks());
     if (s->grid_tiles > (unsigned)kRedCap || s->grid_elem > (unsigned)kRedCap) {
         be_free(s);
         piro::set_error("piro_be_create: reduction grid exceeds %d blocks", kRedCap);
@@ -1924,7 +1967,7 @@ static int be_create(int nx, int ny, int nz, const int32_t *rowptr, const int32_
         s->mdt = -dt;
         s->vself = (float)(-6.0 / (double)norm);
         s->vnb = (float)(1.0 / (double)norm);
-        s->grid_mf = (unsigned)std::min<int64_t>(cdiv(N, kMfThreads), (int64_t)kRedCap);
+        s->grid_mf = (unsigned)std::min<int64_t>(cdiv(N, kMfThreads), mf_blocks());
         int *d_ok = reinterpret_cast<int *>(s->partials);  // scratch before first use
         int h_ok = 0;
         const int one = 1;
@@ -2174,7 +2217,7 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
     double prev_rel = INFINITY;
     for (int outer = 0; outer <= max_outer; ++outer) {
         if (s->op_mf && s->ib_ptr)
-            k_residual_mf<<<(unsigned)std::min<int64_t>(cdiv(N, 256), (int64_t)kRedCap), 256, 0, st>>>(
+            k_residual_mf<<<(unsigned)std::min<int64_t>(cdiv(N, 256), mf_blocks()), 256, 0, st>>>(
                                                               GridDiv(s->nx, s->ny, s->nz), N, s->mdt, s->vself,
                                                               s->vnb, s->ib_ptr, s->ib_col, s->ib_val, s->alpha,
                                                               s->dinv, b, s->x64, s->r, s->z, s->partials, s->st,

@@ -406,6 +406,8 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_conv16_tc(const __grid_cons
             }
         } else {
             // epilogue: warp w holds tile rows 32w .. 32w+31
+            float sc = 1.0f;
+            int64_t sc_of = -1;  // the member whose scale that is
             for (int j = 0; j < P; ++j, tile.next(a)) {
                 const int buf = j % kAcc;
                 if (!mbar_wait(accf(buf), (j / kAcc) & 1, a.err)) break;
@@ -429,8 +431,10 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_conv16_tc(const __grid_cons
                     put_cell(a.out, a.rows, a.cells + lane, make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0));
                 if (kEpi == 1) {
                     if (c < a.N) {
-                        float sc = 1.0f;
-                        if (a.rr) sc = (float)sqrt(a.rr[tile.b] / a.n_int);
+                        if (a.rr && tile.b != sc_of) {  // an FP64 division and root: once per member
+                            sc = (float)sqrt(a.rr[tile.b] / a.n_int);
+                            sc_of = tile.b;
+                        }
                         a.zout[boff + c] = a.g.interior(c) ? __uint_as_float(v[0]) * sc : 0.0f;
                     }
                 } else if (kEpi == 3) {

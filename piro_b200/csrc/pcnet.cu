@@ -511,11 +511,13 @@ __global__ void k_pack_input16(GridDiv g, int64_t N, const float *__restrict__ r
     if (skip && *((volatile const int *)skip)) return;
     const int b = blockIdx.y;
     const int64_t cells = N * gridDim.y, rows = tc::act_rows(cells);
-    float s = 1.0f;
-    if (rr) {
-        const double v = rr[b];
-        s = v > 0.0 ? (float)(1.0 / sqrt(v / n_int)) : 0.0f;
+    __shared__ float s_scale;
+    if (threadIdx.x == 0) {
+        const double v = rr ? rr[b] : 0.0;
+        s_scale = !rr ? 1.0f : v > 0.0 ? (float)(1.0 / sqrt(v / n_int)) : 0.0f;
     }
+    __syncthreads();
+    const float s = s_scale;
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < N; c += (int64_t)gridDim.x * blockDim.x) {
         const int64_t o = (int64_t)b * N + c;
         uint32_t w0 = 0;
