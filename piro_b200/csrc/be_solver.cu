@@ -1303,6 +1303,45 @@ const void *be_resident_kernel(int groups, bool stream_alpha)
     }
 }
 
+// The Jacobi iterations of a learned sweep by the same team, from the state that
+// the network iterations left (U; its scalars from *st) to the sweep's tolerance.
+template <int kK, bool kStreamA>
+__global__ void __launch_bounds__(kRcThreads, 1) k_fcg_resident(RcProblem P, RcResume U, unsigned long long *epoch,
+                                                                RcSlot *slots, DevState *st, long long spin_limit)
+{
+    extern __shared__ float4 s_own[];
+    __shared__ RcShared sh;
+    if (*((volatile int *)&st->done)) return;  // the same in every block: written before this launch
+    const RcTeam T{slots, epoch, (int)blockIdx.x, (int)gridDim.x, &st->bar_err, spin_limit};
+    RcResult R;
+    P.max_inner = st->max_iters;
+    U.tol2 = st->tol2;
+    U.rr0 = st->rr0;
+    U.pq = st->pq;
+    U.iters = st->iters;
+    rc_solve<false, kK, kStreamA, const RcProblem, true>(P, T, sh, s_own, R, U);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        __threadfence();
+        st->iters = R.inner;  // every block has read st before this block's last sums
+        st->rr = R.rel;
+        if (R.status != PIRO_OK) st->broken = 1;
+        st->done = 1;
+    }
+}
+
+const void *fcg_resident_kernel(int groups, bool stream_alpha)
+{
+    switch (cdiv(groups, kRcThreads)) {
+    case 0:
+    case 1: return (const void *)k_fcg_resident<1, false>;
+    case 2: return (const void *)k_fcg_resident<2, false>;
+    case 3: return (const void *)k_fcg_resident<3, false>;
+    case 4:
+    case 5: return (const void *)(stream_alpha ? k_fcg_resident<5, true> : k_fcg_resident<5, false>);
+    default: return (const void *)(stream_alpha ? k_fcg_resident<kRcK, true> : k_fcg_resident<kRcK, false>);
+    }
+}
+
 // The Jacobi iterations of a learned sweep in one cooperative launch: flexible
 // CG (the k_fcg_* iteration above) resumed from the state the network-
 // preconditioned iterations left -- r, the last direction p in p0 and its
@@ -1611,6 +1650,7 @@ struct piro_be_solver {
     size_t res_smem;
     int rc_team;        // k_be_resident: CTAs of the team, 0 if the problem does not fit on chip
     const void *rc_kernel;
+    const void *rc_fcg;  // k_fcg_resident on the same team
     char *rc_mem;       // the rounds' number (256 bytes), the team's slots, the exchange buffer; alpha
     size_t rc_bytes;    // without alpha
     size_t rc_smem;
@@ -1842,9 +1882,12 @@ static int be_setup_persistent(piro_be_solver *s, bool allow_resident)
             static DeviceOnce once;
             int rc2 = device_once(once, dev, []() -> int {
                 for (int groups = kRcThreads; groups <= kRcGroups; groups += kRcThreads)
-                    for (bool sa : {false, true})
+                    for (bool sa : {false, true}) {
                         PIRO_CUDA(cudaFuncSetAttribute(be_resident_kernel(groups, sa),
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
+                        PIRO_CUDA(cudaFuncSetAttribute(fcg_resident_kernel(groups, sa),
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
+                    }
                 return PIRO_OK;
             });
             if (rc2) return rc2;
@@ -1860,6 +1903,9 @@ static int be_setup_persistent(piro_be_solver *s, bool allow_resident)
                 rp.ax = stream ? reinterpret_cast<float4 *>(s->rc_mem + s->rc_bytes) : nullptr;
                 s->rc_problem = rp;
                 s->rc_kernel = kern;
+                const void *fcg = fcg_resident_kernel(rp.groups, stream);
+                PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rc, fcg, kRcThreads, s->rc_smem));
+                s->rc_fcg = per_sm_rc >= 1 ? fcg : nullptr;
                 s->rc_team = team;
             }
         }
@@ -2262,8 +2308,45 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
         while (true) {
             const bool with_net = net_iters;
             net_iters = false;
+            // The rest of the sweep on chip, but for runs of more than five groups per
+            // thread where k_fcg_persistent keeps its vectors on chip as well.  Solves
+            // on B200, on chip / not: 64^3 617 / 742 us, 87 x 64 x 75 741 / 1002, 112^3
+            // (5 groups) 867 / 934, 120^3 (6) 1018 / 1005, 128^3 (7) 1152 / 1142; off
+            // the float4 forms 125 x 127 x 126 (7) 1085 / 1731.
+            const bool beside = s->fcg_res && s->res_cells > 0 && s->nx % 4 == 0 && s->rc_problem.groups > 5 * kRcThreads;
+            if (learned && !with_net && s->persist && s->rc_team > 0 && s->rc_fcg && !beside) {
+                RcProblem Q = s->rc_problem;
+                Q.alpha = s->alpha;
+                Q.mdt = s->mdt;
+                Q.vself = s->vself;
+                Q.vnb = s->vnb;
+                RcResume U{};
+                U.r = s->r;
+                U.p = s->p[kLearnedIters & 1];  // the direction the network iterations left
+                U.q = s->q;
+                U.d = s->d;
+                unsigned long long *epoch = reinterpret_cast<unsigned long long *>(s->rc_mem);
+                RcSlot *slots = reinterpret_cast<RcSlot *>(s->rc_mem + 256);
+                long long spin = wait_limit(1ll << 22);
+                void *rargs[] = {&Q, &U, &epoch, &slots, &s->st, &spin};
+                PIRO_CUDA(cudaMemsetAsync(&s->st->bar_count, 0, 2 * sizeof(unsigned) + sizeof(int), st));
+                PIRO_CUDA(cudaLaunchCooperativeKernel(s->rc_fcg, dim3(s->rc_team), dim3(kRcThreads), rargs, s->rc_smem, st));
+                s->kernel_launches += 1;
+                PIRO_CUDA(cudaMemcpyAsync(s->h_st, s->st, sizeof(DevState), cudaMemcpyDeviceToHost, st));
+                PIRO_CUDA(cudaStreamSynchronize(st));
+                if (s->h_st->bar_err) {
+                    piro::set_error("piro_be_solve: grid barrier timed out");
+                    inf.status = PIRO_ERR_CUDA;
+                    if (info) *info = inf;
+                    // the rounds that slots and exchange buffer hold are not known
+                    PIRO_CUDA(cudaMemsetAsync(s->rc_mem, 0, s->rc_bytes, st));
+                    return PIRO_ERR_CUDA;
+                }
+                seen = s->h_st->iters;
+                break;
+            }
             if (learned && !with_net && s->persist && s->grid_fp > 0) {
-                // the rest of the sweep: Jacobi flexible CG in one cooperative launch
+                // the same in one cooperative launch with two grid barriers per iteration
                 PArgs F{};
                 F.g = GridDiv(s->nx, s->ny, s->nz);
                 F.N = N;

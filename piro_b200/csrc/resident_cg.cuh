@@ -117,6 +117,16 @@ struct RcResult {
     bool ok;  // false: a wait ran out
 };
 
+// A flexible CG iteration to go on with (kResume): its residual, last direction
+// and that direction's A p, the correction so far (read and left), all on the
+// grid; <p, S p>, the iterations so far (0: no direction yet) and the bounds.
+struct RcResume {
+    const float *r, *p, *q;
+    float *d;
+    double tol2, rr0, pq;
+    int iters;
+};
+
 struct RcShared {
     double red[4 * 16];
     double tot[kRcMaxTeam / 32][4];  // per polling warp
@@ -344,8 +354,13 @@ struct RcVec {
 // (with at most kRcRegK, q and d fit in registers beside D, w and p).
 // kStreamA: alpha is read from ax in every iteration.  Prob: the problem by
 // value (a kernel's parameter) or by reference (in shared memory).
-template <bool kConst, int kK, bool kStreamA, class Prob>
-__device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, float4 *smem, RcResult &R)
+// kResume: no refinement sweeps, but the iterations that follow U's up to its
+// tolerance, from the state U on.  Its first direction is conjugate to U's p, and
+// its residual orthogonal to p, as a CG iteration leaves them; from then on they are
+// CG iterations.  R.inner counts U's iterations too, R.rel is |r|^2.
+template <bool kConst, int kK, bool kStreamA, class Prob, bool kResume = false>
+__device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, float4 *smem, RcResult &R,
+                                         const RcResume U = RcResume())
 {
     constexpr bool kReg = kK <= kRcRegK;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -398,7 +413,7 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
         sh.halo = 0;
     }
     // boundary cells: x = b; x64 = 0, or b for constant alpha (its residual reads them)
-    {
+    if (!kResume) {
         const int total = P.ny * P.nz, w = tid >> 5, nw = kRcThreads / 32;
 #pragma unroll 1
         for (int ln = T.rank * nw + w; ln < total; ln += T.size * nw) {
@@ -470,7 +485,7 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
         }
     __syncthreads();
     // beff: the two ends of every line, then the lines next to a face
-    if (!kConst) {
+    if (!kConst && !kResume) {
         auto fold = [&](int64_t i) {
             double be = (double)__ldg(P.b + i);
 #pragma unroll 1
@@ -502,6 +517,34 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
             d.put(k, v, zero);
         }
     }
+    if (kResume) {  // U's p, q / alpha (by way of z's memory) and d
+        auto stage = [&](float *to, const float *from, bool over_alpha) {
+            __syncthreads();
+#pragma unroll 1
+            for (int c = tid; c < 4 * ng; c += kRcThreads) {
+                int x, y, z;
+                const bool in = where(c, x, y, z);
+                const float v = from[cell(x, y, z)], a = __ldg(P.alpha + cell(x, y, z));
+                to[c] = in ? over_alpha ? v / a : v : 0.0f;
+            }
+            __syncthreads();
+        };
+        if (U.iters > 0) {
+            stage(szf, U.p, false);
+#pragma unroll
+            for (int k = 0; k < kK; ++k)
+                if (tid + k * kRcThreads < ng) p[k] = sz[tid + k * kRcThreads];
+            stage(szf, U.q, true);
+#pragma unroll
+            for (int k = 0; k < kK; ++k)
+                if (tid + k * kRcThreads < ng) q.put(k, tid + k * kRcThreads, sz[tid + k * kRcThreads]);
+        }
+        stage(sdf, U.d, false);
+        if (kReg)
+#pragma unroll
+            for (int k = 0; k < kK; ++k)
+                if (tid + k * kRcThreads < ng) d.put(k, 0, d.s[tid + k * kRcThreads]);
+    }
     unsigned long long tag = T.size > 1 ? *((volatile unsigned long long *)T.epoch) : 0;
     unsigned round = (unsigned)tag, flip = 0;  // round: of z, never ahead of tag
     R.status = PIRO_ERR_NOT_CONVERGED;
@@ -523,6 +566,22 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
         // R: r = b - A x in FP64, z = s / D, a cell per thread (coalesced).
         // Sweep 0 has x = b, read from b itself.
         double rs[4] = {0.0, 0.0, 0.0, 0.0};
+        if (kResume) {  // U's r; <s, z> and <z, S p> of its direction
+#pragma unroll 1
+            for (int c = tid; c < 4 * ng; c += kRcThreads) {
+                int x, y, z;
+                const bool here = where(c, x, y, z);
+                const int64_t i = cell(x, y, z);
+                const float a = __ldg(P.alpha + i), rf = U.r[i], qf = U.iters > 0 ? U.q[i] : 0.0f;
+                const float c32 = __fadd_rn(1.0f, __fmul_rn(P.mdt, __fmul_rn(a, P.vself)));
+                const float zz = here ? rf * rcp_approx(c32) : 0.0f;
+                if (here) {
+                    rs[2] += (double)(rf * rcp_approx(a)) * (double)zz;
+                    rs[1] += (double)zz * (double)qf / (double)a;
+                }
+                szf[c] = zz;
+            }
+        } else
 #pragma unroll 1
         for (int c = tid; c < 4 * ng; c += kRcThreads) {
             int x, y, z;
@@ -568,6 +627,15 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
             for (int v = tid; v < ng; v += kRcThreads) send(v, (int)P.fgx.div((uint32_t)v), sz[v]);
         if (!rc_allreduce(T, sh, kRcWordR, 4, tag, rs[0], rs[1], rs[2], rs[3], false)) { R.ok = false; return; }
         const double rt[4] = {sh.out[0], sh.out[1], sh.out[2], sh.out[3]};
+        double tol2 = U.tol2, rr0 = U.rr0, beta0 = 0.0, rz = rt[2], pq = 0.0;
+        if (kResume) {
+            R.status = PIRO_OK;
+            R.inner = U.iters;
+            if (U.iters > 0) {
+                pq = U.pq;
+                beta0 = -rt[1] / pq;
+            }
+        } else {
         const double bn = rt[1] > 0.0 ? sqrt(rt[1]) : 1.0;
         R.rel = sqrt(rt[0]) / bn;
         if (!isfinite(R.rel)) { R.status = PIRO_STATUS_STALLED; break; }
@@ -579,12 +647,13 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
         double itol = 0.5 * P.rtol / R.rel;
         itol = itol > 0.1 ? 0.1 : itol;
         itol = itol < P.inner_floor ? P.inner_floor : itol;
-        const double tol2 = itol * itol, rr0 = rt[3];
-        double rz = rt[2], pq = 0.0;
+        tol2 = itol * itol;
+        rr0 = rt[3];
+        }
         double sum[3] = {0.0, 0.0, 0.0};  // this thread's <s, z>, <z, w>, |alpha s|^2
-        bool first = true, broken = false;
+        bool first = true, broken = kResume && !isfinite(beta0);
 #pragma unroll 1
-        while (rr0 > 0.0) {
+        while (rr0 > 0.0 && !broken) {
             // H: the halo's lines, two words per group, as they arrive
             if (T.size > 1) {
                 const int nh = sh.halo * gx;
@@ -643,11 +712,12 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
                 return;
             }
             const double st[3] = {sh.out[0], sh.out[1], sh.out[2]};
-            double beta = 0.0;
+            double beta = beta0;
             if (!first) {
                 ++R.inner;
                 beta = st[0] / rz;
                 rz = st[0];
+                if (kResume) R.rel = st[2];
                 if (!isfinite(st[2]) || !isfinite(beta)) { broken = !kConst; break; }
                 if (st[2] <= tol2 * rr0 || R.inner >= P.max_inner) break;
             }
@@ -688,7 +758,8 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
             }
             if (kConst) sum[2] *= (double)P.alpha0 * (double)P.alpha0;
         }
-        if (broken && !kConst) { R.status = PIRO_STATUS_STALLED; break; }
+        if (broken && !kConst) R.status = PIRO_STATUS_STALLED;
+        if (broken && !kConst && !kResume) break;
         // X: x += d, a cell per thread (d through shared memory)
         if (kReg) {
 #pragma unroll
@@ -709,23 +780,27 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
                 int x, y, z;
                 in[j] = where(c0 + j * kRcThreads, x, y, z);
                 ci[j] = cell(x, y, z);
-                if (sweep > 0) xo[j] = P.x64[ci[j]];
+                if (kResume) xo[j] = 0.0;
+                else if (sweep > 0) xo[j] = P.x64[ci[j]];
                 else xo[j] = (double)__ldg(P.b + ci[j]);
             }
 #pragma unroll
             for (int j = 0; j < kB; ++j) {
                 const int c = c0 + j * kRcThreads;
                 if (c >= 4 * ng) break;
-                if (in[j]) P.x64[ci[j]] = xo[j] + (double)sdf[c];
+                if (kResume && in[j]) U.d[ci[j]] = sdf[c];
+                else if (in[j]) P.x64[ci[j]] = xo[j] + (double)sdf[c];
                 if (!kReg) sdf[c] = 0.0f;
             }
         }
+        if (kResume) break;
         if (broken) { R.status = PIRO_STATUS_STALLED; break; }  // constant alpha: ends with the correction it has
         // every CTA's x64 before the next residual reads its neighbours
         ++tag;
         if (!rc_allreduce(T, sh, kRcWordX, 1, tag, 0.0, 0.0, 0.0, 0.0, true)) { R.ok = false; return; }
     }
     if (T.size > 1 && T.rank == 0 && tid == 0) *T.epoch = tag;  // every CTA has read it before its first sums
+    if (kResume) return;
     // the interior from x64 (b itself if no sweep ran)
 #pragma unroll 1
     for (int c = tid; c < 4 * ng; c += kRcThreads) {
