@@ -1650,7 +1650,7 @@ struct piro_be_solver {
     size_t res_smem;
     int rc_team;        // k_be_resident: CTAs of the team, 0 if the problem does not fit on chip
     const void *rc_kernel;
-    const void *rc_fcg;  // k_fcg_resident on the same team
+    const void *rc_fcg;  // k_fcg_resident on the same team, from the first learned solve on
     char *rc_mem;       // the rounds' number (256 bytes), the team's slots, the exchange buffer; alpha
     size_t rc_bytes;    // without alpha
     size_t rc_smem;
@@ -1879,18 +1879,8 @@ static int be_setup_persistent(piro_be_solver *s, bool allow_resident)
         RcProblem rp = rc_geometry(s->nx, s->ny, s->nz, team);
         if (rc_fits(rp, false, stream)) {
             const void *kern = be_resident_kernel(rp.groups, stream);
-            static DeviceOnce once;
-            int rc2 = device_once(once, dev, []() -> int {
-                for (int groups = kRcThreads; groups <= kRcGroups; groups += kRcThreads)
-                    for (bool sa : {false, true}) {
-                        PIRO_CUDA(cudaFuncSetAttribute(be_resident_kernel(groups, sa),
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
-                        PIRO_CUDA(cudaFuncSetAttribute(fcg_resident_kernel(groups, sa),
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
-                    }
-                return PIRO_OK;
-            });
-            if (rc2) return rc2;
+            // this instance alone: every other one would be loaded as well
+            PIRO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
             int per_sm_rc = 0;
             s->rc_smem = rc_smem(rp, false, stream);
             PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rc, kern, kRcThreads, s->rc_smem));
@@ -1903,9 +1893,6 @@ static int be_setup_persistent(piro_be_solver *s, bool allow_resident)
                 rp.ax = stream ? reinterpret_cast<float4 *>(s->rc_mem + s->rc_bytes) : nullptr;
                 s->rc_problem = rp;
                 s->rc_kernel = kern;
-                const void *fcg = fcg_resident_kernel(rp.groups, stream);
-                PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rc, fcg, kRcThreads, s->rc_smem));
-                s->rc_fcg = per_sm_rc >= 1 ? fcg : nullptr;
                 s->rc_team = team;
             }
         }
@@ -2314,7 +2301,14 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
             // (5 groups) 867 / 934, 120^3 (6) 1018 / 1005, 128^3 (7) 1152 / 1142; off
             // the float4 forms 125 x 127 x 126 (7) 1085 / 1731.
             const bool beside = s->fcg_res && s->res_cells > 0 && s->nx % 4 == 0 && s->rc_problem.groups > 5 * kRcThreads;
-            if (learned && !with_net && s->persist && s->rc_team > 0 && s->rc_fcg && !beside) {
+            const bool on_chip = learned && !with_net && s->persist && s->rc_team > 0 && !beside;
+            if (on_chip && !s->rc_fcg) {
+                // one CTA per SM, as k_be_resident: the same threads, registers and shared memory at most
+                const void *fcg = fcg_resident_kernel(s->rc_problem.groups, s->rc_problem.ax != nullptr);
+                PIRO_CUDA(cudaFuncSetAttribute(fcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
+                s->rc_fcg = fcg;
+            }
+            if (on_chip) {
                 RcProblem Q = s->rc_problem;
                 Q.alpha = s->alpha;
                 Q.mdt = s->mdt;
