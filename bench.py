@@ -657,7 +657,8 @@ def batched_section(torch, ops, peak, steps=4):
         "error_vs_fp64": {"be_members_checked": len(errs_be), "be_max_rel_err": max(errs_be) if errs_be else None,
                           "fe_members_bitexact": f"{fe_ok}/{fe_n}"},
         "note": "one cooperative launch per step (two steps per CUDA graph); bytes counted per member from its "
-                "CG iterations and refinement sweeps",
+                "CG iterations and refinement sweeps as if they came from HBM: the grouped schedule keeps a "
+                "member's vectors on chip, so the figure may exceed the HBM peak",
     }
 
 
@@ -765,15 +766,15 @@ def run_piro(args):
     ck = main["clocks"]
     x = torch.empty_like(u0)
     # roofline of the dominant kernel (the one persistent launch per step):
-    # what binds it is latency -- L2 round trips of the neighbour reads and
-    # the grid barriers of each CG iteration -- not HBM (its data stay in L2
-    # and shared memory between phases).  achieved/frac: DRAM bytes per launch
+    # what binds it is latency -- one all-reduce over L2 and the halo lines of
+    # each CG iteration, and its shared-memory phases -- not HBM (its vectors
+    # stay on chip).  achieved/frac: DRAM bytes per launch
     # (the committed ncu capture of the same 128^3 launch) / event-timed
     # duration against the copy peak; binding: the L2-throughput and
     # issue-slot fractions of that capture; effective: the CG bytes of the
     # CSR formulation (8 nnz + 4(N+1) + 60 N per iteration, 8 nnz + 4(N+1) +
     # 24 N per FP64 residual) over the same time.
-    k_name = "k_be_persistent" if inner_op == "stencil-persistent" else (
+    k_name = "k_be_resident" if inner_op == "stencil-persistent" else (
         "k_cg_spmv_mf" if inner_op == "stencil" else "k_cg_spmv")
     avg_spmv_ms = main["spmv_ms"] / max(1, main["spmv_launches"])
     prof = profiled_metrics(k_name)
@@ -790,19 +791,19 @@ def run_piro(args):
         "frac": None if dram_gbs is None else round(dram_gbs / peak, 4), "peak_kind": peak_kind,
         "traffic": traffic, "avg_launch_ms": avg_spmv_ms, "launches": main["spmv_launches"],
         "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum per launch, ncu capture of the same "
-                          "128^3 launch (profiles/k_be_persistent_128.md)",
+                          "128^3 launch (profiles/k_be_resident_128.md)",
         "binding": {"l2_throughput_frac": (prof["lts__throughput.avg.pct_of_peak_sustained_elapsed"] / 100
                                            if "lts__throughput.avg.pct_of_peak_sustained_elapsed" in prof else None),
                     "issue_active_frac": (prof["smsp__issue_active.avg.pct_of_peak_sustained_active"] / 100
                                           if "smsp__issue_active.avg.pct_of_peak_sustained_active" in prof else None),
                     "us_per_cg_iteration": round(1e3 * avg_spmv_ms / max(main["iters"], 1e-9), 2),
-                    "note": "latency bound: L2 round trips of neighbour reads and two grid all-reduces per CG "
-                            "iteration; DRAM moves only the step's first touch of its data"},
+                    "note": "latency bound: one all-reduce over L2 and the neighbours' halo lines per CG iteration, "
+                            "vectors on chip; DRAM moves only the step's first touch of its data"},
         "effective": {"bytes_per_launch": eff_bytes, "gbs": round(eff_bytes / avg_spmv_ms / 1e6, 1),
                       "frac_of_hbm_peak": round(eff_bytes / avg_spmv_ms / 1e6 / peak, 4),
                       "note": "algorithmic bytes of the CSR formulation (per CG iteration 8 nnz + 4(N+1) + 60 N, "
                               "per FP64 residual 8 nnz + 4(N+1) + 24 N); this kernel is matrix-free and serves "
-                              "them from L2 and shared memory, so the figure exceeds the HBM peak"},
+                              "them from shared memory and L2, so the figure exceeds the HBM peak"},
     }
 
     # end to end through host buffers: every step copies u_n from pinned host

@@ -2224,7 +2224,8 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
             s->persist_ms += ms;
             s->persist_launches += 1;
             // algorithmic bytes: P0 32, residual sweep 32 + update 24, CG iteration 8 (phase A: z, alpha)
-            // + 12 (phase B: z, alpha in, z out) bytes per cell (the resident form; p, d, q stay on chip)
+            // + 12 (phase B: z, alpha in, z out) bytes per cell (k_be_persistent with p, d, q on chip; k_be_resident
+            // keeps z there as well)
             const double n = (double)N;
             s->persist_bytes += n * (32.0 + 56.0 * (s->h_st->p_outer + 1) + 20.0 * s->h_st->p_inner + 8.0);
         } else {
