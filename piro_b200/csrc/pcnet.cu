@@ -356,20 +356,32 @@ __global__ void __launch_bounds__(256) k_conv_bwd_w(GridDiv g, int64_t N, int B,
     }
 }
 
-// out[p] = sum over blocks (fixed order, FP64) of partials[block][p].  Bound by
-// the latency of the loads, 32 of them at a time: 148 partials of 6912 values take
-// 17 us, four at a time they took 22 (B200).
-__global__ void __launch_bounds__(64) k_reduce_partials(const float *__restrict__ partials, int nblocks, int P, float *__restrict__ out)
+// out[p] = sum over blocks (fixed order, FP64) of partials[block][p]: kRedSegs
+// threads per value add a stretch of the blocks each, 16 loads at a time, and the
+// first of them adds the stretches.  Bound by latency: 148 partials of 6912 values
+// take 5 us; one thread per value took 17 with 32 loads at a time and 22 with
+// four (B200).
+constexpr int kRedSegs = 8;
+
+__global__ void __launch_bounds__(32 * kRedSegs) k_reduce_partials(const float *__restrict__ partials, int nblocks, int P,
+                                                                   float *__restrict__ out)
 {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int k0 = 0; k0 < nblocks; k0 += 32) {
-            float v[32];
+    __shared__ double s_seg[kRedSegs][32];
+    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+    const int each = (nblocks + kRedSegs - 1) / kRedSegs, b0 = seg * each, b1 = min(b0 + each, nblocks);
+    double s = 0.0;
+    if (p < P)
+        for (int k0 = b0; k0 < b1; k0 += 16) {
+            float v[16];
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = partials[(int64_t)(k0 + k < nblocks ? k0 + k : nblocks - 1) * P + p];
+            for (int k = 0; k < 16; ++k) v[k] = __ldg(partials + (int64_t)(k0 + k < b1 ? k0 + k : b1 - 1) * P + p);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) s += k0 + k < nblocks ? (double)v[k] : 0.0;  // + 0: s is never -0
+            for (int k = 0; k < 16; ++k) s += k0 + k < b1 ? (double)v[k] : 0.0;  // + 0: s is never -0
         }
+    s_seg[seg][lane] = s;
+    __syncthreads();
+    if (seg == 0 && p < P) {
+        for (int q = 1; q < kRedSegs; ++q) s += s_seg[q][lane];
         out[p] = (float)s;
     }
 }
@@ -803,7 +815,7 @@ static int launch_wgrad_tc(piro_pcnet *n, const GridDiv &g, int64_t cells, const
     tc::k_wgrad_tc<<<(unsigned)grid, tc::kWgThreads, tc::kWgSmemBytes, st>>>(xmap, gmap, a);
     PIRO_CHECK_LAUNCH("k_wgrad_tc");
     const int P = kTaps * CI * CO;
-    k_reduce_partials<<<(P + 63) / 64, 64, 0, st>>>(n->partials, (int)grid, P, grad_w);
+    k_reduce_partials<<<(P + 31) / 32, 32 * kRedSegs, 0, st>>>(n->partials, (int)grid, P, grad_w);
     PIRO_CHECK_LAUNCH("k_reduce_partials");
     n->launches += 2;
     return PIRO_OK;
@@ -826,7 +838,7 @@ static int launch_bwd_w(piro_pcnet *n, const GridDiv &g, int64_t N, int batch, c
     const int nblocks = kRedBlocks;
     constexpr int P = kTaps * CI * CO;
     k_conv_bwd_w<CI, CO, GT><<<nblocks, 256, smem, st>>>(g, N, batch, x, gy, n->partials);
-    k_reduce_partials<<<(P + 63) / 64, 64, 0, st>>>(n->partials, nblocks, P, grad_w);
+    k_reduce_partials<<<(P + 31) / 32, 32 * kRedSegs, 0, st>>>(n->partials, nblocks, P, grad_w);
     n->launches += 2;
     PIRO_CHECK_LAUNCH("k_conv_bwd_w");
     return PIRO_OK;
