@@ -423,19 +423,34 @@ __global__ void k_finish_sum(double *red, int slot)
 
 // Masked MSE: loss = sum m (out - t)^2 / sum m; gout = 2 m (out - t) / sum m
 // on interior cells (boundary outputs are constant zeros: gout = 0 there).
-__global__ void __launch_bounds__(256) k_loss(GridDiv g, int64_t N, int64_t n, const float *__restrict__ out,
+// kPlanes: gout as the 16-channel BF16 planes of the tensor-core layers, channel 0
+// = bf16(gout) and the rest 0, with the rows after the last cell.  fN: division
+// by N for n < 2^31.
+template <bool kPlanes>
+__global__ void __launch_bounds__(256) k_loss(GridDiv g, int64_t N, FastDiv fN, int64_t n, const float *__restrict__ out,
                                               const float *__restrict__ tgt, const float *__restrict__ mask,
-                                              double *__restrict__ red, float *__restrict__ gout)
+                                              double *__restrict__ red, float *__restrict__ gout, bf16 *__restrict__ g16)
 {
     __shared__ double sw[32];
     const double msum = red[kRedBlocks + 0];
     const float inv = msum > 0.0 ? (float)(1.0 / msum) : 0.0f;
     double s = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float d = out[i] - tgt[i];
-        const float m = mask[i];
-        s += (double)m * (double)d * (double)d;
-        gout[i] = g.interior(i % N) ? 2.0f * m * d * inv : 0.0f;
+    const int64_t rows = kPlanes ? tc::act_rows(n) : n;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
+        float go = 0.0f;
+        if (i < n) {
+            const float d = out[i] - tgt[i];
+            const float m = mask[i];
+            s += (double)m * (double)d * (double)d;
+            const int64_t c = n < ((int64_t)1 << 31) ? i - (int64_t)fN.div((uint32_t)i) * N : i % N;
+            go = g.interior(c) ? 2.0f * m * d * inv : 0.0f;
+        }
+        if (kPlanes) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(go, 0.0f);
+            tc::put_cell(g16, rows, i, make_uint4(*reinterpret_cast<const uint32_t *>(&h), 0, 0, 0), make_uint4(0, 0, 0, 0));
+        } else {
+            gout[i] = go;
+        }
     }
     s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = s;
@@ -499,18 +514,6 @@ __global__ void k_pack_wtc_t(const float *__restrict__ wq, Layout L, bf16 *__res
         const int CI = l == 0 ? 2 : 16, CO = l == kLayers - 1 ? 1 : 16;
         const float v = (gin < CO && gout < CI) ? wq[L.w[l] + ((kTaps - 1 - tap) * CI + gout) * CO + gin] : 0.0f;
         wpk_t[i] = __float2bfloat16_rn(v);
-    }
-}
-
-// The loss gradient (FP32, one channel) as a 16-channel BF16 array: channel 0
-// = bf16(gout), the rest 0 -- the input of the last layer's data gradient and
-// weight gradient on the tensor cores.
-__global__ void k_pack_grad16(int64_t n, const float *__restrict__ gout, bf16 *__restrict__ g16)
-{
-    const int64_t rows = tc::act_rows(n);  // zeros from n on
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(i < n ? gout[i] : 0.0f, 0.0f);
-        tc::put_cell(g16, rows, i, make_uint4(*reinterpret_cast<const uint32_t *>(&h), 0, 0, 0), make_uint4(0, 0, 0, 0));
     }
 }
 
@@ -1028,7 +1031,11 @@ extern "C" int piro_pcnet_loss_grad(piro_pcnet *n, int batch, int nx, int ny, in
     if (rc) return rc;
     k_mask_sum<<<kRedBlocks, 256, 0, st>>>(cells, mask, n->red);
     k_finish_sum<<<1, 320, 0, st>>>(n->red, 0);
-    k_loss<<<kRedBlocks, 256, 0, st>>>(g, N, cells, n->out, target, mask, n->red, n->gout);
+    const FastDiv fN((uint32_t)N);
+    if (tcore)
+        k_loss<true><<<kRedBlocks, 256, 0, st>>>(g, N, fN, cells, n->out, target, mask, n->red, nullptr, n->go16);
+    else
+        k_loss<false><<<kRedBlocks, 256, 0, st>>>(g, N, fN, cells, n->out, target, mask, n->red, n->gout, nullptr);
     k_finish_sum<<<1, 320, 0, st>>>(n->red, 1);
     PIRO_CHECK_LAUNCH("k_loss");
     const dim3 grid(net_grid(N, 128), batch);
@@ -1036,8 +1043,6 @@ extern "C" int piro_pcnet_loss_grad(piro_pcnet *n, int batch, int nx, int ny, in
         // backward on the tensor cores: per layer the weight gradient (GEMM over
         // the cells), then the data gradient into the previous layer's
         // pre-activation (transposed, tap-reversed convolution times GELU')
-        k_pack_grad16<<<net_grid(cells, 256), 256, 0, st>>>(cells, n->gout, n->go16);
-        PIRO_CHECK_LAUNCH("k_pack_grad16");
         rc = launch_wgrad_tc(n, g, cells, n->a[2], n->go16, 16, 1, n->g + L.w[3], st);
         if (!rc)
             rc = conv_tc<3>(n->go16, n->g16[0], nullptr, n->wpk_t + 2 * W, g, N, batch, nullptr, 0.0, nullptr,
@@ -1052,7 +1057,7 @@ extern "C" int piro_pcnet_loss_grad(piro_pcnet *n, int batch, int nx, int ny, in
                             nullptr, n->y[0]);
         if (!rc) rc = launch_wgrad_tc(n, g, cells, n->x16, n->g16[0], 2, 16, n->g + L.w[0], st);
         if (rc) return rc;
-        n->launches += 4;
+        n->launches += 3;
         if (loss) {
             PIRO_CUDA(cudaMemcpyAsync(loss, n->red + kRedBlocks + 1, sizeof(double), cudaMemcpyDeviceToHost, st));
         }
