@@ -124,6 +124,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
         : "memory");
     return ok != 0;
 }
+// Programmatic dependent launch: the next kernel's blocks may come as this one's
+// leave; a kernel waits for the one before it after its own set-up, before it
+// reads or writes anything of the layers.  (The weights are packed two launches or
+// more ahead.)  One training step's gradients, 18 launches: 485 us without, 429
+// with (16 crops of 34^3, B200).
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Bounded wait for the phase with the given parity; false on timeout or when
 // another role already gave up.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err)
@@ -295,7 +303,10 @@ __device__ __forceinline__ void put_zero(const Args &a, int64_t c)
 template <int kEpi>
 __global__ void __launch_bounds__(kThreads, kCtas) k_conv16_tc(const __grid_constant__ CUtensorMap xmap, Args a)
 {
-    if (a.skip && *((volatile const int *)a.skip)) return;
+    if (a.skip) {
+        grid_wait();
+        if (*((volatile const int *)a.skip)) return;
+    }
     extern __shared__ unsigned char smem_raw[];
     unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
     const uint32_t planes_s = smem_u32(sm);
@@ -343,6 +354,8 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_conv16_tc(const __grid_cons
     fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(tmem_slot), 0);
 
+    grid_launch_next();
+    grid_wait();
     if (P > 0) {
         if (warp == 4) {
             if (lane == 0) {

@@ -367,6 +367,8 @@ __global__ void __launch_bounds__(32 * kRedSegs) k_reduce_partials(const float *
                                                                    float *__restrict__ out)
 {
     __shared__ double s_seg[kRedSegs][32];
+    tc::grid_launch_next();
+    tc::grid_wait();
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
     const int each = (nblocks + kRedSegs - 1) / kRedSegs, b0 = seg * each, b1 = min(b0 + each, nblocks);
     double s = 0.0;
@@ -732,6 +734,21 @@ static int encode_rows_map(CUtensorMap *m, const void *base, int64_t cells)
     return PIRO_OK;
 }
 
+// A launch whose blocks may start their set-up while the kernel before it ends.
+static cudaLaunchConfig_t overlap_launch(cudaLaunchAttribute *at, unsigned grid, unsigned threads, size_t smem, cudaStream_t st)
+{
+    at->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at->val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return c;
+}
+
 // One layer on the tensor cores over `batch` grids of N cells: in (16 BF16
 // channels per cell) -> out (GELU, 16 BF16 channels) or, for the last layer,
 // zout (FP32 channel 0 times sqrt(rr / n_int)).  Every cell of the output is
@@ -758,7 +775,9 @@ static int conv_tc(const bf16 *in, bf16 *out, float *zout, const bf16 *wpk, cons
     const int64_t ntiles = (int64_t)batch * ncol * (g.nz - 2);
     const int64_t grid = ntiles < tc::kCtas * sm_count() ? ntiles : tc::kCtas * sm_count();
     tc::Args a{g, N, nxy, ntiles, ncol, wpk, out, zout, rr, n_int, skip, err, N * batch, tc::act_rows(N * batch), yout, yprev};
-    tc::k_conv16_tc<kEpi><<<(unsigned)grid, tc::kThreads, tc::kSmemBytes, st>>>(map, a);
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t lc = overlap_launch(&at, (unsigned)grid, tc::kThreads, tc::kSmemBytes, st);
+    PIRO_CUDA(cudaLaunchKernelEx(&lc, tc::k_conv16_tc<kEpi>, map, a));
     PIRO_CHECK_LAUNCH("k_conv16_tc");
     return PIRO_OK;
 }
@@ -815,10 +834,13 @@ static int launch_wgrad_tc(piro_pcnet *n, const GridDiv &g, int64_t cells, const
     if (grid > kRedBlocks) grid = kRedBlocks;
     if (grid > ntiles) grid = ntiles;
     tc::WgArgs a{g.nx, (int64_t)g.nx * g.ny, ntiles, CI, CO, n->partials, n->d_err};
-    tc::k_wgrad_tc<<<(unsigned)grid, tc::kWgThreads, tc::kWgSmemBytes, st>>>(xmap, gmap, a);
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t lc = overlap_launch(&at, (unsigned)grid, tc::kWgThreads, tc::kWgSmemBytes, st);
+    PIRO_CUDA(cudaLaunchKernelEx(&lc, tc::k_wgrad_tc, xmap, gmap, a));
     PIRO_CHECK_LAUNCH("k_wgrad_tc");
     const int P = kTaps * CI * CO;
-    k_reduce_partials<<<(P + 31) / 32, 32 * kRedSegs, 0, st>>>(n->partials, (int)grid, P, grad_w);
+    const cudaLaunchConfig_t lr = overlap_launch(&at, (P + 31) / 32, 32 * kRedSegs, 0, st);
+    PIRO_CUDA(cudaLaunchKernelEx(&lr, k_reduce_partials, (const float *)n->partials, (int)grid, P, grad_w));
     PIRO_CHECK_LAUNCH("k_reduce_partials");
     n->launches += 2;
     return PIRO_OK;

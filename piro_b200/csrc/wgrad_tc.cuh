@@ -106,6 +106,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_tc(const __grid_constan
     fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(tmem_slot), 0);
     bool mma_ok = my_tiles > 0;
+    grid_launch_next();
+    grid_wait();
 
     if (warp == 4) {
         if (lane == 0 && my_tiles > 0) {
