@@ -553,6 +553,7 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
     R.rel = INFINITY;
     R.ok = true;
     double prev_rel = INFINITY;
+    bool corrected = false;  // x64 holds a sweep's result
     auto send = [&](int v, int ll, const float4 &z4) {
         const int n = nat[ll];
         if (n < 0) {
@@ -793,6 +794,7 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
                 if (!kReg) sdf[c] = 0.0f;
             }
         }
+        corrected = true;
         if (kResume) break;
         if (broken) { R.status = PIRO_STATUS_STALLED; break; }  // constant alpha: ends with the correction it has
         // every CTA's x64 before the next residual reads its neighbours
@@ -801,14 +803,14 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
     }
     if (T.size > 1 && T.rank == 0 && tid == 0) *T.epoch = tag;  // every CTA has read it before its first sums
     if (kResume) return;
-    // the interior from x64 (b itself if no sweep ran)
+    // the interior from x64 (b itself if no sweep came to its end)
 #pragma unroll 1
     for (int c = tid; c < 4 * ng; c += kRcThreads) {
         int x, y, z;
         if (!where(c, x, y, z)) continue;
         const int64_t i = cell(x, y, z);
-        const double xv = R.outer > 0 ? P.x64[i] : (double)P.b[i];
-        if (R.outer == 0) P.x64[i] = xv;
+        const double xv = corrected ? P.x64[i] : (double)P.b[i];
+        if (!corrected) P.x64[i] = xv;
         P.xout[i] = (float)xv;
     }
 }
