@@ -40,6 +40,7 @@
 // remains, and gives the same bits).  The solve (one block, FP64) replays the
 // exchanges and Gauss transforms on b and back-substitutes.
 #include "common.cuh"
+#include "lu_order.cuh"
 
 namespace piro {
 namespace {
@@ -701,7 +702,9 @@ __global__ void __launch_bounds__(256) k_lupb_update(int64_t N, int64_t bw, int6
 //
 // Columns: a block owns the strips of 8 columns s with 1 + s mod (blocks - 1)
 // equal to it, in every panel, so that it only waits for block 0 (a ready
-// counter) and block 0 only for the two strips it takes over next.  A strip's
+// counter) and block 0 only for the two strips it takes over next.  A block may
+// lag by any number of panels otherwise: what it reads of a panel (Lp, the pivots,
+// which give the row order) is not written again.  A strip's
 // 16 pivot rows are substituted by shuffles, then one pass applies the 16 steps
 // to the rows below in order.  The blocks also store the panel's multipliers
 // to the band: from the panel's threads, a row each, these stores alone cost
@@ -712,7 +715,7 @@ __global__ void __launch_bounds__(256) k_lupb_update(int64_t N, int64_t bw, int6
 // (864 panels of 592 rows) 23.3 ms, against 74.6 by three launches per panel
 // with the panel in shared memory and three barriers a step; 12^3 2.1 against
 // 7.1, 24 x 24 x 6 5.9 against 18.3 (B200).  Block 0 per panel, in thousands of
-// cycles: the steps 35, Lp and the row order out 5, the next columns' pivot rows
+// cycles: the steps 35, Lp out 5, the next columns' pivot rows
 // 2 and update 10.  Waits are bounded.
 constexpr int kLuPanelRows = 736;  // 512 threads, with 128 registers each
 constexpr int kLuStrip = 8;
@@ -720,12 +723,10 @@ constexpr int kLuHelp = 128;  // block 0's threads that fetch and publish
 constexpr int kLuLd = kLuNbMax + 1;
 constexpr int kLuShare = 8;  // rows of multipliers a block stores at a time
 constexpr int kLuThreads = kLuPanelRows / 2 + 16 + kLuHelp;  // two rows per thread, in whole warps
-constexpr int kLuPerms = 8;  // panels whose row order is kept
 
 struct LuSync {
     unsigned ready;  // panels factored
     unsigned urgent; // strips applied that are the next panel but one
-    unsigned done;   // blocks x panels applied
     int timeout;
 };
 
@@ -733,7 +734,6 @@ struct LuArgs {
     int64_t N, bw, W;
     double *band, *Lc, *Lp;
     int32_t *piv;
-    int *perm;  // [kLuPerms][bw + 16]
     int *err;
     LuSync *sync;
     long long spin_limit;
@@ -883,10 +883,11 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
             // the first strip at or after `first` that this block owns
             int64_t st = first + (((int64_t)blockIdx.x - 1 - first) % nb + nb) % nb;
             const double *lp = A.Lp + (int64_t)pi * kLuNbMax * ldl;
-            if (tid < kLuNbMax) s_piv[tid] = tid < nbp ? __ldcg(A.piv + j0 + tid) - (int)j0 : 0;
+            if (tid < kLuNbMax) s_piv[tid] = tid < nbp ? __ldcg(A.piv + j0 + tid) - (int)j0 : tid;
+            __syncthreads();
+            for (int r = tid; r < R; r += blockDim.x) s_perm[r] = lu_row_before(s_piv, 0, kLuNbMax, r);
             if (st <= last) {
                 for (int r = tid; r < R; r += blockDim.x) {
-                    s_perm[r] = __ldcg(A.perm + (pi % kLuPerms) * ldl + r);
 #pragma unroll
                     for (int k = 0; k < kLuNbMax; ++k) {
                         const double l = __ldcg(lp + k * ldl + r);
@@ -908,19 +909,10 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
             if (tid < kLuShare * kLuNbMax) {
                 const int k = tid % kLuNbMax;
                 for (int r = (int)blockIdx.x - 1 + nb * (tid / kLuNbMax); r < R; r += nb * kLuShare) {
-                    int q = r;
-                    if (r < nbp || __ldcg(A.perm + (pi % kLuPerms) * ldl + r) != r)
-#pragma unroll 1
-                        for (int kk = nbp - 1; kk > k; --kk) {
-                            const int pk = s_piv[kk];
-                            if (q == kk) q = pk;
-                            else if (q == pk) q = kk;
-                        }
+                    const int q = r < nbp || s_perm[r] != r ? lu_row_before(s_piv, k + 1, nbp, r) : r;
                     if (k < nbp && k < r && q - k <= bw) *band_at(A.band, W, bw, j0 + q, j0 + k) = __ldcg(lp + (int64_t)k * ldl + r);
                 }
             }
-            __syncthreads();
-            if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&A.sync->done) : "memory");
         }
         return;
     }
@@ -945,15 +937,12 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
             const int64_t j0 = (int64_t)pi * kLuNbMax, j1 = j0 + kLuNbMax;
             sync_on(kFree, all);
             if (pi + 1 < npan) {
-                // The next panel's columns, once the strips of the last panel are in
-                // them; and that panel's slot for its row order, once it is read.
+                // The next panel's columns, once the strips of the last panel are in them.
                 if (ht == 0) {
                     const int64_t cl = j0 - kLuNbMax + kLuNbMax - 1 + 2 * bw < N - 1 ? j0 - 1 + 2 * bw : N - 1;  // the last panel's last column
                     const int64_t left = pi > 0 ? cl / kLuStrip - j1 / kLuStrip + 1 : 0;
                     due += left > kLuNbMax / kLuStrip ? kLuNbMax / kLuStrip : left > 0 ? (unsigned)left : 0u;
-                    const unsigned old = pi + 1 >= kLuPerms ? (unsigned)(pi + 2 - kLuPerms) * (gridDim.x - 1) : 0u;
-                    const bool ok = lu_poll(A, &A.sync->urgent, due) && lu_poll(A, &A.sync->done, old);
-                    if (!ok) s_flag = 0;
+                    if (!lu_poll(A, &A.sync->urgent, due)) s_flag = 0;
                     asm volatile("fence.acq_rel.gpu;" ::: "memory");
                 }
                 sync_on(kHelpBar, kLuHelp);
@@ -1120,7 +1109,6 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
             for (int h = 0; h < 2; ++h) {
                 const int r = p0 + h;
                 if (r >= R) continue;
-                A.perm[(pi % kLuPerms) * ldl + r] = rid[h];
                 s_perm[r] = rid[h];
                 if (r < nbp) {
 #pragma unroll
@@ -1726,9 +1714,8 @@ __global__ void __launch_bounds__(kPreThreads, 1) k_lup_solve_pre(int64_t N, int
 
 // Device layout of the factor buffer: band double[N][3bw+1], Lc double[N][bw],
 // y double[N] (the solve's workspace), piv int32[N], err int[2] and LuSync, Lw
-// double[bw + 16][16] (the launched panels' multipliers) or perm int[2][bw + 16]
-// (k_lupb_factor's exchanges), Lp double[ceil(N/16)][16][bw + 16] (the solve's
-// panel multipliers).
+// double[bw + 16][16] (the launched panels' multipliers), Lp
+// double[ceil(N/16)][16][bw + 16] (the solve's panel multipliers).
 struct LupLayout {
     int64_t W;
     size_t band, lc, y, piv, err, lw, lp, total;  // byte offsets
@@ -1857,7 +1844,6 @@ extern "C" int piro_ht_lu_factor(int64_t N, int64_t bw, const int64_t *keys, con
         A.Lc = Lc;
         A.Lp = reinterpret_cast<double *>(base + L.lp);
         A.piv = piv;
-        A.perm = reinterpret_cast<int *>(base + L.lw);
         A.err = err;
         A.sync = reinterpret_cast<LuSync *>(base + L.err + 64);
         A.spin_limit = wait_limit(1ll << 22);  // ~2 s of polling per wait
