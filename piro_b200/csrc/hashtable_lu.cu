@@ -724,8 +724,10 @@ constexpr int kLuLd = kLuNbMax + 1;
 constexpr int kLuShare = 8;  // rows of multipliers a block stores at a time
 constexpr int kLuThreads = kLuPanelRows / 2 + 16 + kLuHelp;  // two rows per thread, in whole warps
 
+constexpr unsigned kLuStop = 0x7fffffffu;  // in place of the count: a singular column, no panel follows
+
 struct LuSync {
-    unsigned ready;  // panels factored
+    unsigned ready;  // panels factored, or kLuStop
     unsigned urgent; // strips applied that are the next panel but one
     int timeout;
 };
@@ -739,15 +741,14 @@ struct LuArgs {
     long long spin_limit;
 };
 
-// Waits until *count >= want; false if it ran out.  The caller orders what
-// follows by a fence: an acquire per poll would empty L1 each time.
-__device__ __forceinline__ bool lu_poll(const LuArgs &A, const unsigned *count, unsigned want)
+// Waits until *count >= want, left in seen; false if it ran out.  The caller orders
+// what follows by a fence: an acquire per poll would empty L1 each time.
+__device__ __forceinline__ bool lu_poll(const LuArgs &A, const unsigned *count, unsigned want, unsigned &seen)
 {
     long long spins = 0;
     while (true) {
-        unsigned c;
-        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
-        if (c >= want) return true;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+        if (seen >= want) return true;
         if (++spins > A.spin_limit || *((volatile int *)&A.sync->timeout)) {
             atomicExch(&A.sync->timeout, 1);
             return false;
@@ -755,11 +756,15 @@ __device__ __forceinline__ bool lu_poll(const LuArgs &A, const unsigned *count, 
     }
 }
 
-// Thread 0 waits; the result in every thread.
-__device__ __forceinline__ bool lu_wait(const LuArgs &A, const unsigned *count, unsigned want, int *s_flag)
+// Thread 0 waits for panel want - 1; false in every thread if the wait ran out or
+// block 0 has stopped.  It stops once every block has applied the panel before the
+// singular one to the columns it waits for, so a block must not leave sooner, on
+// the error flag for instance.
+__device__ __forceinline__ bool lu_wait(const LuArgs &A, unsigned want, int *s_flag)
 {
     if (threadIdx.x == 0) {
-        *s_flag = lu_poll(A, count, want) ? 1 : 0;
+        unsigned seen = 0;
+        *s_flag = lu_poll(A, &A.sync->ready, want, seen) && seen != kLuStop ? 1 : 0;
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
     }
     __syncthreads();
@@ -876,8 +881,7 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
         for (int pi = 0; pi < npan; ++pi) {
             const int64_t j0 = (int64_t)pi * kLuNbMax;
             const int nbp = (int)(N - j0 < kLuNbMax ? N - j0 : kLuNbMax), R = rows_of(j0, nbp);
-            if (!lu_wait(A, &A.sync->ready, (unsigned)pi + 1, &s_flag)) return;
-            if (*((volatile int *)A.err)) return;
+            if (!lu_wait(A, (unsigned)pi + 1, &s_flag)) return;
             const int64_t cmax = j0 + nbp - 1 + 2 * bw < N - 1 ? j0 + nbp - 1 + 2 * bw : N - 1;
             const int64_t first = (j0 + 2 * kLuNbMax) / kLuStrip, last = cmax / kLuStrip;
             // the first strip at or after `first` that this block owns
@@ -942,7 +946,8 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
                     const int64_t cl = j0 - kLuNbMax + kLuNbMax - 1 + 2 * bw < N - 1 ? j0 - 1 + 2 * bw : N - 1;  // the last panel's last column
                     const int64_t left = pi > 0 ? cl / kLuStrip - j1 / kLuStrip + 1 : 0;
                     due += left > kLuNbMax / kLuStrip ? kLuNbMax / kLuStrip : left > 0 ? (unsigned)left : 0u;
-                    if (!lu_poll(A, &A.sync->urgent, due)) s_flag = 0;
+                    unsigned seen = 0;
+                    if (!lu_poll(A, &A.sync->urgent, due, seen)) s_flag = 0;
                     asm volatile("fence.acq_rel.gpu;" ::: "memory");
                 }
                 sync_on(kHelpBar, kLuHelp);
@@ -973,7 +978,7 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lupb_factor(LuArgs A)
             if (!s_flag) return;
             if (ht == 0) {
                 __threadfence();
-                atomicExch(&A.sync->ready, s_stop ? 0x7fffffffu : (unsigned)pi + 1);  // stop: every waiter sees err
+                atomicExch(&A.sync->ready, s_stop ? kLuStop : (unsigned)pi + 1);
             }
             if (s_stop) return;
         }
@@ -1834,6 +1839,7 @@ extern "C" int piro_ht_lu_factor(int64_t N, int64_t bw, const int64_t *keys, con
     if (ub && ub[0] == '1') nb = 0;
     // One launch where the panel's rows fit in block 0's registers and the panel
     // reaches columns past the next one (bw >= 16); the launches below otherwise.
+    LuSync hsync{};
     bool one_launch = nb == kLuNbMax && bw >= kLuNbMax && bw + kLuNbMax <= kLuPanelRows;
     if (one_launch) {
         LuArgs A;
@@ -1868,13 +1874,7 @@ extern "C" int piro_ht_lu_factor(int64_t N, int64_t bw, const int64_t *keys, con
             PIRO_CUDA(cudaMemsetAsync(A.sync, 0, sizeof(LuSync), st));
             void *args[] = {&A};
             PIRO_CUDA(cudaLaunchCooperativeKernel((const void *)k_lupb_factor, dim3(grid), dim3(threads), args, smem, st));
-            LuSync h;
-            PIRO_CUDA(cudaMemcpyAsync(&h, A.sync, sizeof(LuSync), cudaMemcpyDeviceToHost, st));
-            PIRO_CUDA(cudaStreamSynchronize(st));
-            if (h.timeout) {
-                set_error("piro_ht_lu_factor: a wait between blocks timed out");
-                return PIRO_ERR_CUDA;
-            }
+            PIRO_CUDA(cudaMemcpyAsync(&hsync, A.sync, sizeof(LuSync), cudaMemcpyDeviceToHost, st));
         }
     }
     if (one_launch) {
@@ -1913,6 +1913,10 @@ extern "C" int piro_ht_lu_factor(int64_t N, int64_t bw, const int64_t *keys, con
     if (herr[0] == 3) {
         set_error("piro_ht_lu_factor: singular matrix: column %d has no nonzero at or below the diagonal", herr[1]);
         return PIRO_ERR_ZERO_PIVOT;
+    }
+    if (hsync.timeout) {  // after err: a singular column is the answer, whatever else gave up
+        set_error("piro_ht_lu_factor: a wait between blocks timed out");
+        return PIRO_ERR_CUDA;
     }
     if (one_launch) return PIRO_OK;  // Lp is written
     const int64_t lp_items = cdiv(N, kLuSolveNb) * (bw + kLuSolveNb) * kLuSolveNb;

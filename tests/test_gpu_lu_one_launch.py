@@ -82,3 +82,17 @@ def test_lu_one_launch_wait_gives_up(cuda):
         lib().piro_set_wait_limit(-1)
     for got, ref in zip(_parts(ops.HtLu(300, 60, keys, vals, ts, 0.0, 1.0), 300, 60), want):
         assert np.array_equal(got, ref)
+
+
+def test_lu_one_launch_singular_beside_a_wait_that_gave_up(cuda):
+    """A zero first column, found without a wait, while the other blocks' first wait gives up."""
+    from piro_b200 import ops
+    from piro_b200._lib import PiroError, lib
+    (keys, vals), ts, _ = _table(ops, 100, 20, 5, 0)
+    assert lib().piro_set_wait_limit(0) == 0
+    try:
+        with pytest.raises(PiroError, match="column 0 ") as e:
+            ops.HtLu(100, 20, keys, vals, ts, 0.0, 1.0)
+        assert e.value.status == 12  # PIRO_ERR_ZERO_PIVOT
+    finally:
+        lib().piro_set_wait_limit(-1)
