@@ -35,6 +35,7 @@
 // on timeout an error flag is raised and every block leaves.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include "common.cuh"
@@ -60,10 +61,13 @@ struct BState {
     double rz, rr0, tol2, rel, prev_rel, a, beta;
 };
 
+// count, gen and active are set to zero before every launch that uses them, err only
+// at the start of a call: a wait that ran out in one of its launches is still seen
+// after the last, and the launches behind it leave at their first wait.
 struct BarrierState {
     unsigned count, gen;
-    int err;
     int active[2];
+    int err;
 };
 
 struct BArgs {
@@ -837,6 +841,9 @@ __global__ void __launch_bounds__(kRcThreads, 1) k_batch_resident(RArgs A)
     extern __shared__ float4 s_own[];
     __shared__ RcShared sh;
     __shared__ RJob J;
+    // After a launch whose wait ran out the slots and the exchange buffers hold words of
+    // rounds that this one would number again.  One thread's reading, for the whole block.
+    if (__syncthreads_or(threadIdx.x == 0 && *((volatile int *)&A.bar->err))) return;
     // forward-Euler members: one pass over their tiles by every CTA
     for (int t = blockIdx.x; t < A.nfe; t += gridDim.x) {
         const BMember m = A.mem[A.fe_tile_m[t]];
@@ -1394,7 +1401,6 @@ static int batch_launch_groups(piro_batch *s, const float *u, float *out, cudaSt
     A.max_inner = 20000;
     A.spin_limit = wait_limit(1ll << 22);  // ~2 s of polling per barrier wait
     void *args[] = {&A};
-    PIRO_CUDA(cudaMemsetAsync(s->bar, 0, sizeof(BarrierState), st));
     PIRO_CUDA(cudaMemsetAsync(s->d_job_bar, 0, sizeof(unsigned) * (size_t)std::max(1, s->njobs), st));
     PIRO_CUDA(cudaLaunchCooperativeKernel((const void *)k_batch_groups, dim3(s->grid_g), dim3(kThreads), args, 0, st));
     return PIRO_OK;
@@ -1421,7 +1427,6 @@ static int batch_launch_resident(piro_batch *s, const float *u, float *out, cuda
     A.max_inner = 20000;
     A.spin_limit = wait_limit(1ll << 22);  // ~2 s of polling per wait
     void *args[] = {&A};
-    PIRO_CUDA(cudaMemsetAsync(s->bar, 0, sizeof(BarrierState), st));
     PIRO_CUDA(cudaLaunchCooperativeKernel((const void *)k_batch_resident, dim3(s->grid_g), dim3(kRcThreads), args,
                                           s->r_smem, st));
     return PIRO_OK;
@@ -1459,8 +1464,8 @@ static int batch_launch(piro_batch *s, const float *u, float *out, cudaStream_t 
     A.max_rounds = 40000;
     A.spin_limit = wait_limit(1ll << 22);  // ~2 s of polling per barrier wait
     void *args[] = {&A};
-    // a launch whose barrier wait gave up leaves count, gen and err behind
-    PIRO_CUDA(cudaMemsetAsync(s->bar, 0, sizeof(BarrierState), st));
+    // a launch whose barrier wait gave up leaves count and gen behind
+    PIRO_CUDA(cudaMemsetAsync(s->bar, 0, offsetof(BarrierState, err), st));
     PIRO_CUDA(cudaLaunchCooperativeKernel(batch_kernel(s->blocks_per_sm), dim3(s->grid), dim3(kThreads), args, 0, st));
     return PIRO_OK;
 }
@@ -1496,6 +1501,21 @@ static int batch_pair_graph(piro_batch *s)
     return PIRO_OK;
 }
 
+// Before the launches of a call, and after them (the stream idle): whether a wait ran out.
+static int batch_clear_err(piro_batch *s)
+{
+    PIRO_CUDA(cudaMemsetAsync(&s->bar->err, 0, sizeof(int), s->stream));
+    return PIRO_OK;
+}
+
+static int batch_take_err(piro_batch *s, int *err)
+{
+    PIRO_CUDA(cudaMemcpy(err, &s->bar->err, sizeof(int), cudaMemcpyDeviceToHost));
+    // the rounds that slots and exchange buffers hold are not known
+    if (*err && s->d_rjobs) PIRO_CUDA(cudaMemsetAsync(s->r_mem, 0, s->r_bytes > 0 ? s->r_bytes : 256, s->stream));
+    return PIRO_OK;
+}
+
 extern "C" int piro_batch_step(piro_batch *s, int steps, double rtol, double *ms)
 {
     PIRO_ARG(s && steps >= 0 && rtol > 0.0, "piro_batch_step: bad arguments");
@@ -1505,27 +1525,28 @@ extern "C" int piro_batch_step(piro_batch *s, int steps, double rtol, double *ms
         int rc = batch_pair_graph(s);
         if (rc) return rc;
     }
+    int rc = batch_clear_err(s);
+    if (rc) return rc;
     PIRO_CUDA(cudaEventRecord(s->e0, s->stream));
     if (s->cur == 1 && k < steps) {  // realign to f[0] so the pair graph applies
-        int rc = batch_launch(s, s->f[1], s->f[0], s->stream);
+        rc = batch_launch(s, s->f[1], s->f[0], s->stream);
         if (rc) return rc;
         s->cur = 0;
         ++k;
     }
     for (; k + 2 <= steps; k += 2) PIRO_CUDA(cudaGraphLaunch(s->pair, s->stream));
     if (k < steps) {
-        int rc = batch_launch(s, s->f[0], s->f[1], s->stream);
+        rc = batch_launch(s, s->f[0], s->f[1], s->stream);
         if (rc) return rc;
         s->cur = 1;
     }
     PIRO_CUDA(cudaEventRecord(s->e1, s->stream));
     PIRO_CUDA(cudaStreamSynchronize(s->stream));
-    BarrierState hb;
-    PIRO_CUDA(cudaMemcpy(&hb, s->bar, sizeof(hb), cudaMemcpyDeviceToHost));
-    if (hb.err) {
+    int err = 0;
+    rc = batch_take_err(s, &err);
+    if (rc) return rc;
+    if (err) {
         set_error("piro_batch_step: grid barrier timed out");
-        // the rounds that slots and exchange buffers hold are not known
-        if (s->d_rjobs) PIRO_CUDA(cudaMemset(s->r_mem, 0, s->r_bytes > 0 ? s->r_bytes : 256));
         return PIRO_ERR_CUDA;
     }
     float t = 0.0f;
@@ -1550,6 +1571,25 @@ extern "C" int piro_batch_member_info(piro_batch *s, int *status, int *sweeps, i
     return PIRO_OK;
 }
 
+// The time of one step from the current fields, its result discarded (the second of
+// two); infinite if a wait ran out.
+static int batch_time_step(piro_batch *s, float *ms)
+{
+    int rc = batch_clear_err(s);
+    for (int rep = 0; rep < 2 && !rc; ++rep) {
+        PIRO_CUDA(cudaEventRecord(s->e0, s->stream));
+        rc = batch_launch(s, s->f[s->cur], s->f[s->cur ^ 1], s->stream);
+        if (rc) return rc;
+        PIRO_CUDA(cudaEventRecord(s->e1, s->stream));
+        PIRO_CUDA(cudaStreamSynchronize(s->stream));
+        PIRO_CUDA(cudaEventElapsedTime(ms, s->e0, s->e1));
+    }
+    int err = 0;
+    if (!rc) rc = batch_take_err(s, &err);
+    if (err) *ms = INFINITY;
+    return rc;
+}
+
 // Autotuner: time one step (from the current fields, result discarded) for
 // each tile size and blocks-per-SM candidate of the lockstep step and for the
 // grouped step at 2 and 4 CTAs per SM, and keep the fastest.
@@ -1568,14 +1608,8 @@ extern "C" int piro_batch_autotune(piro_batch *s, double rtol, int *tile_out, in
             if (rc) return rc;
             if (s->blocks_per_sm != b) continue;  // occupancy does not allow it
             float ms = INFINITY;
-            for (int rep = 0; rep < 2; ++rep) {  // second run timed
-                PIRO_CUDA(cudaEventRecord(s->e0, s->stream));
-                rc = batch_launch(s, s->f[s->cur], s->f[s->cur ^ 1], s->stream);
-                if (rc) return rc;
-                PIRO_CUDA(cudaEventRecord(s->e1, s->stream));
-                PIRO_CUDA(cudaStreamSynchronize(s->stream));
-                PIRO_CUDA(cudaEventElapsedTime(&ms, s->e0, s->e1));
-            }
+            rc = batch_time_step(s, &ms);
+            if (rc) return rc;
             if (ms < best) {
                 best = ms;
                 bt = t;
@@ -1592,18 +1626,9 @@ extern "C" int piro_batch_autotune(piro_batch *s, double rtol, int *tile_out, in
         if (s->d_rjobs) b = 1;  // one CTA per SM, whatever is asked for
         s->grouped = 1;
         float ms = INFINITY;
-        for (int rep = 0; rep < 2; ++rep) {
-            PIRO_CUDA(cudaEventRecord(s->e0, s->stream));
-            rc = batch_launch(s, s->f[s->cur], s->f[s->cur ^ 1], s->stream);
-            if (rc) {
-                s->grouped = 0;
-                return rc;
-            }
-            PIRO_CUDA(cudaEventRecord(s->e1, s->stream));
-            PIRO_CUDA(cudaStreamSynchronize(s->stream));
-            PIRO_CUDA(cudaEventElapsedTime(&ms, s->e0, s->e1));
-        }
+        rc = batch_time_step(s, &ms);
         s->grouped = 0;
+        if (rc) return rc;
         if (ms < best) {
             best = ms;
             bg = b;
@@ -1619,6 +1644,10 @@ extern "C" int piro_batch_autotune(piro_batch *s, double rtol, int *tile_out, in
         batch_free_groups(s);
     }
     batch_drop_graph(s);
+    if (!std::isfinite(best)) {
+        set_error("piro_batch_autotune: grid barrier timed out in every candidate");
+        return PIRO_ERR_CUDA;
+    }
     if (tile_out) *tile_out = bt;
     if (blocks_per_sm_out) *blocks_per_sm_out = bb;
     return PIRO_OK;

@@ -77,3 +77,31 @@ def test_grouped_waits_give_up(cuda):
     B.step(1)
     assert np.array_equal(B.get_fields(), want)
     B.close()
+
+
+@pytest.mark.parametrize("steps", [2, 3, "autotune"])
+def test_grouped_waits_give_up_in_any_launch(cuda, steps):
+    """Several launches whose waits give up, in one call: the call says so, and nothing
+    of their rounds is taken for a later launch's (other fields, so that it would show)."""
+    from piro_b200._lib import PiroError, lib
+    B, u0, n, sc = _batch((40, 33, 20, 9), (1, 1, 0, 1))
+    B.set_schedule(True, 2)
+    u1 = np.ascontiguousarray(u0[::-1])
+    B.set_fields(u1)
+    B.step(3)
+    want = B.get_fields()
+    B.set_fields(u0)
+    try:
+        assert lib().piro_set_wait_limit(0) == 0
+        with pytest.raises(PiroError) as e:
+            B.autotune(1e-8) if steps == "autotune" else B.step(steps)
+        assert e.value.status == 6 and "timed out" in str(e.value)
+    finally:
+        lib().piro_set_wait_limit(-1)
+    B.set_schedule(True, 2) if steps == "autotune" else None
+    B.set_fields(u1)
+    B.step(3)
+    got = B.get_fields()
+    for k in range(len(n)):  # the cells between the members belong to none
+        assert np.array_equal(B.member(got, k), B.member(want, k)), k
+    B.close()
