@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(kRcThreads, 1) k_batch_resident(RArgs A)
         __syncthreads();
         const RcTeam T{J.slots, J.epoch, (int)blockIdx.x - J.gbase, J.gsize, &A.bar->err, A.spin_limit};
         RcResult R;
-        rc_solve<true, kRcK, false, const RcProblem &>(J.P, T, sh, s_own, R);
+        rc_solve<true, kRcK, false, false, const RcProblem &>(J.P, T, sh, s_own, R);
         if (T.rank == 0 && threadIdx.x == 0) {
             BState s{};
             s.mode = kDone;

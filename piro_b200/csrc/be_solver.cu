@@ -1271,7 +1271,7 @@ __global__ void __launch_bounds__(kPT, 2) k_be_persistent(PArgs P)
 
 // The whole solve by one team of CTAs with z, p, q, d of their lines in shared
 // memory (resident_cg.cuh).
-template <int kK, bool kStreamA>
+template <int kK, bool kStreamA, bool kWide>
 __global__ void __launch_bounds__(kRcThreads, 1) k_be_resident(RcProblem P,
                                                                unsigned long long *epoch, RcSlot *slots,
                                                                DevState *st, long long spin_limit)
@@ -1280,7 +1280,7 @@ __global__ void __launch_bounds__(kRcThreads, 1) k_be_resident(RcProblem P,
     __shared__ RcShared sh;
     const RcTeam T{slots, epoch, (int)blockIdx.x, (int)gridDim.x, &st->bar_err, spin_limit};
     RcResult R;
-    rc_solve<false, kK, kStreamA, const RcProblem>(P, T, sh, s_own, R);
+    rc_solve<false, kK, kStreamA, kWide, const RcProblem>(P, T, sh, s_own, R);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->p_status = R.ok ? R.status : PIRO_ERR_CUDA;
         st->p_outer = R.outer;
@@ -1290,22 +1290,23 @@ __global__ void __launch_bounds__(kRcThreads, 1) k_be_resident(RcProblem P,
 }
 
 // The instance for a run of at most `groups` groups.
+template <bool kWide>
 const void *be_resident_kernel(int groups, bool stream_alpha)
 {
     switch (cdiv(groups, kRcThreads)) {
     case 0:
-    case 1: return (const void *)k_be_resident<1, false>;
-    case 2: return (const void *)k_be_resident<2, false>;
-    case 3: return (const void *)k_be_resident<3, false>;
+    case 1: return (const void *)k_be_resident<1, false, kWide>;
+    case 2: return (const void *)k_be_resident<2, false, kWide>;
+    case 3: return (const void *)k_be_resident<3, false, kWide>;
     case 4:
-    case 5: return (const void *)(stream_alpha ? k_be_resident<5, true> : k_be_resident<5, false>);
-    default: return (const void *)(stream_alpha ? k_be_resident<kRcK, true> : k_be_resident<kRcK, false>);
+    case 5: return (const void *)(stream_alpha ? k_be_resident<5, true, kWide> : k_be_resident<5, false, kWide>);
+    default: return (const void *)(stream_alpha ? k_be_resident<kRcK, true, kWide> : k_be_resident<kRcK, false, kWide>);
     }
 }
 
 // The Jacobi iterations of a learned sweep by the same team, from the state that
 // the network iterations left (U; its scalars from *st) to the sweep's tolerance.
-template <int kK, bool kStreamA>
+template <int kK, bool kStreamA, bool kWide>
 __global__ void __launch_bounds__(kRcThreads, 1) k_fcg_resident(RcProblem P, RcResume U, unsigned long long *epoch,
                                                                 RcSlot *slots, DevState *st, long long spin_limit)
 {
@@ -1319,7 +1320,7 @@ __global__ void __launch_bounds__(kRcThreads, 1) k_fcg_resident(RcProblem P, RcR
     U.rr0 = st->rr0;
     U.pq = st->pq;
     U.iters = st->iters;
-    rc_solve<false, kK, kStreamA, const RcProblem, true>(P, T, sh, s_own, R, U);
+    rc_solve<false, kK, kStreamA, kWide, const RcProblem, true>(P, T, sh, s_own, R, U);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         __threadfence();
         st->iters = R.inner;  // every block has read st before this block's last sums
@@ -1329,16 +1330,17 @@ __global__ void __launch_bounds__(kRcThreads, 1) k_fcg_resident(RcProblem P, RcR
     }
 }
 
+template <bool kWide>
 const void *fcg_resident_kernel(int groups, bool stream_alpha)
 {
     switch (cdiv(groups, kRcThreads)) {
     case 0:
-    case 1: return (const void *)k_fcg_resident<1, false>;
-    case 2: return (const void *)k_fcg_resident<2, false>;
-    case 3: return (const void *)k_fcg_resident<3, false>;
+    case 1: return (const void *)k_fcg_resident<1, false, kWide>;
+    case 2: return (const void *)k_fcg_resident<2, false, kWide>;
+    case 3: return (const void *)k_fcg_resident<3, false, kWide>;
     case 4:
-    case 5: return (const void *)(stream_alpha ? k_fcg_resident<5, true> : k_fcg_resident<5, false>);
-    default: return (const void *)(stream_alpha ? k_fcg_resident<kRcK, true> : k_fcg_resident<kRcK, false>);
+    case 5: return (const void *)(stream_alpha ? k_fcg_resident<5, true, kWide> : k_fcg_resident<5, false, kWide>);
+    default: return (const void *)(stream_alpha ? k_fcg_resident<kRcK, true, kWide> : k_fcg_resident<kRcK, false, kWide>);
     }
 }
 
@@ -1878,7 +1880,11 @@ static int be_setup_persistent(piro_be_solver *s, bool allow_resident)
         bool stream = false;
         RcProblem rp = rc_geometry(s->nx, s->ny, s->nz, team);
         if (rc_fits(rp, false, stream)) {
-            const void *kern = be_resident_kernel(rp.groups, stream);
+            // the sums' terms as k_be_persistent takes them on this grid
+            const bool al16 = ((reinterpret_cast<uintptr_t>(s->alpha) | reinterpret_cast<uintptr_t>(s->dinv)) & 15) == 0;
+            rp.wide_u = !(N % 4 == 0 && al16);
+            rp.wide_s = rp.wide_u || s->nx % 4 != 0;
+            const void *kern = rp.wide_s ? be_resident_kernel<true>(rp.groups, stream) : be_resident_kernel<false>(rp.groups, stream);
             // this instance alone: every other one would be loaded as well
             PIRO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
             int per_sm_rc = 0;
@@ -2305,7 +2311,9 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
             const bool on_chip = learned && !with_net && s->persist && s->rc_team > 0 && !beside;
             if (on_chip && !s->rc_fcg) {
                 // one CTA per SM, as k_be_resident: the same threads, registers and shared memory at most
-                const void *fcg = fcg_resident_kernel(s->rc_problem.groups, s->rc_problem.ax != nullptr);
+                const RcProblem &rp = s->rc_problem;
+                const void *fcg = rp.wide_s ? fcg_resident_kernel<true>(rp.groups, rp.ax != nullptr)
+                                            : fcg_resident_kernel<false>(rp.groups, rp.ax != nullptr);
                 PIRO_CUDA(cudaFuncSetAttribute(fcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
                 s->rc_fcg = fcg;
             }

@@ -25,6 +25,13 @@
 // Against the two all-reduces of the usual form one L2 round trip less is
 // exposed, and the vectors pass through shared memory once, not twice.
 //
+// The sums' terms.  Where the launch with grid barriers takes the operator's and
+// the update's dot products in groups of four cells (nx, and nx ny nz, a multiple
+// of 4) their terms are FP32 products, four added in FP32; elsewhere each is an
+// FP64 product (wide_s, wide_u), so that fields of 1e-25 or 1e20, whose FP32
+// products vanish or overflow, are solved there.  <p, S p> by the recurrence below
+// differs from the sum over the cells by what CG's orthogonality has lost.
+//
 // Lines are ordered in strips of h planes (y within a strip, z within h
 // fastest), so that a run of consecutive lines is about square in (y, z) and
 // most of its neighbours are its own.  A table gives for every line where its
@@ -101,6 +108,7 @@ struct RcProblem {
     const float *ib_val;
     double rtol, inner_floor;
     int max_outer, max_inner;
+    int wide_s, wide_u;  // FP64 terms in S and in U (read by the kWide instances alone)
 };
 
 struct RcTeam {
@@ -346,19 +354,30 @@ struct RcVec {
     }
 };
 
+// The sum of a group's four products, each in FP64 (wide) or all in FP32.
+template <bool kWide>
+__device__ __forceinline__ double rc_dot(const float4 &a, const float4 &b, bool wide)
+{
+    if (kWide && wide)
+        return ((double)a.x * (double)b.x + (double)a.y * (double)b.y) + ((double)a.z * (double)b.z + (double)a.w * (double)b.w);
+    return (double)((a.x * b.x + a.y * b.y) + (a.z * b.z + a.w * b.w));
+}
+
 // Solve A x = b for one problem on this CTA's team.  Every CTA of the team
 // runs it with the same arguments and takes the same branches.  kConst:
 // constant alpha (the batched members: boundary neighbours enter the residual
 // with their own value and the stencil's coefficient); else alpha per cell,
 // and the interior-boundary block of A from ib_*.  kK: groups per thread
 // (with at most kRcRegK, q and d fit in registers beside D, w and p).
-// kStreamA: alpha is read from ax in every iteration.  Prob: the problem by
+// kStreamA: alpha is read from ax in every iteration.  kWide: the sums' terms as
+// P.wide_s and P.wide_u say, else FP32 products (an instance of its own: the other
+// widths keep their registers).  Prob: the problem by
 // value (a kernel's parameter) or by reference (in shared memory).
 // kResume: no refinement sweeps, but the iterations that follow U's up to its
 // tolerance, from the state U on.  Its first direction is conjugate to U's p, and
 // its residual orthogonal to p, as a CG iteration leaves them; from then on they are
 // CG iterations.  R.inner counts U's iterations too, R.rel is |r|^2.
-template <bool kConst, int kK, bool kStreamA, class Prob, bool kResume = false>
+template <bool kConst, int kK, bool kStreamA, bool kWide, class Prob, bool kResume = false>
 __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, float4 *smem, RcResult &R,
                                          const RcResume U = RcResume())
 {
@@ -577,7 +596,7 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
                 const float c32 = __fadd_rn(1.0f, __fmul_rn(P.mdt, __fmul_rn(a, P.vself)));
                 const float zz = here ? rf * rcp_approx(c32) : 0.0f;
                 if (here) {
-                    rs[2] += (double)(rf * rcp_approx(a)) * (double)zz;
+                    rs[2] += (double)rf / (double)a * (double)zz;
                     rs[1] += (double)zz * (double)qf / (double)a;
                 }
                 szf[c] = zz;
@@ -615,7 +634,7 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
             if (here) {
                 rs[0] += ri * ri;
                 rs[1] += bi * bi;
-                rs[2] += (double)(rf * rcp_approx(a)) * (double)zz;
+                rs[2] += (double)rf / (double)a * (double)zz;
                 rs[3] += (double)rf * (double)rf;
             }
             szf[c] = zz;
@@ -703,7 +722,7 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
                         if (lx < 3) w[k].z = 0.0f;
                         if (lx < 4) w[k].w = 0.0f;
                     }
-                    sum[1] += (double)((zc.x * w[k].x + zc.y * w[k].y) + (zc.z * w[k].z + zc.w * w[k].w));
+                    sum[1] += rc_dot<kWide>(zc, w[k], kWide && P.wide_s);
                 }
             }
             ++tag;
@@ -752,9 +771,9 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
                     d.put(k, v, dd);
                     sz[v] = zn;
                     if (T.size > 1) send(v, ll, zn);
-                    sum[0] += (double)((s.x * zn.x + s.y * zn.y) + (s.z * zn.z + s.w * zn.w));
+                    sum[0] += rc_dot<kWide>(s, zn, kWide && P.wide_u);
                     if (!kConst) { s.x *= al.x; s.y *= al.y; s.z *= al.z; s.w *= al.w; }
-                    sum[2] += (double)((s.x * s.x + s.y * s.y) + (s.z * s.z + s.w * s.w));
+                    sum[2] += rc_dot<kWide>(s, s, kWide && P.wide_u);
                 }
             }
             if (kConst) sum[2] *= (double)P.alpha0 * (double)P.alpha0;
