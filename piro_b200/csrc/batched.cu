@@ -1048,8 +1048,11 @@ static int batch_resident_setup(piro_batch *s)
         J.off = m.off;
         J.P = rc_geometry(m.g.nx, m.g.nx, m.g.nx, J.gsize);
         if (!fits(J.P)) return PIRO_OK;  // a larger team's strips can need more halo: keep the other kernel
-        J.P.alpha0 = m.alpha;
-        J.P.mdt = -m.dt;
+        // alpha 2^-e in [1/2, 1) and dt 2^e: the same operator, while the solver's vectors
+        // r / alpha stay near r (with alpha itself, 1e-12, fields above 1e7 overflowed)
+        int e = 0;
+        J.P.alpha0 = std::frexp(m.alpha, &e);
+        J.P.mdt = -std::ldexp(m.dt, e);
         J.P.vself = -6.0f;
         J.P.vnb = 1.0f;
         J.P.cd64 = m.cd64;

@@ -634,11 +634,12 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
             if (here) {
                 rs[0] += ri * ri;
                 rs[1] += bi * bi;
-                rs[2] += (double)rf / (double)a * (double)zz;
+                rs[2] += (kConst ? (double)rf : (double)rf / (double)a) * (double)zz;
                 rs[3] += (double)rf * (double)rf;
             }
             szf[c] = zz;
         }
+        if (kConst) rs[2] /= (double)P.alpha0;
         ++tag;
         ++round;
         __syncthreads();
@@ -828,8 +829,9 @@ __device__ __forceinline__ void rc_solve(Prob P, const RcTeam T, RcShared &sh, f
         int x, y, z;
         if (!where(c, x, y, z)) continue;
         const int64_t i = cell(x, y, z);
-        const double xv = corrected ? P.x64[i] : (double)P.b[i];
-        if (!corrected) P.x64[i] = xv;
+        const bool have = kConst ? R.outer > 0 : corrected;  // a sweep begun is a sweep ended for constant alpha
+        const double xv = have ? P.x64[i] : (double)P.b[i];
+        if (!have) P.x64[i] = xv;
         P.xout[i] = (float)xv;
     }
 }

@@ -36,3 +36,29 @@ def test_scaled_field(cuda, n, flexible, exponent):
     diff = (y.double() * 2.0 ** -exponent - x.double()).abs().max()
     assert float(diff) <= 1e-6 * float(x.abs().max())
     s.close()
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+def test_batch_member_of_small_alpha(cuda, grouped):
+    """alpha 2^-40 of another member's with dt 2^40 of its: the operator is the same, and
+    so is the field, bit for bit, at any size of the field."""
+    import numpy as np
+    from piro_b200 import ops
+    n = np.array([20, 20, 33, 33], np.int32)
+    f = 2.0 ** np.array([0, -40, 0, -40])
+    alpha, dt = (0.01 * f).astype(np.float32), (830.0 / f).astype(np.float32)
+    B = ops.Batch(n, alpha, dt, np.ones(4, np.int32))
+    B.set_schedule(grouped, 2)
+    rng = np.random.default_rng(5)
+    u = np.zeros(B.total, np.float32)
+    for k in (0, 2):
+        v = rng.random(int(n[k]) ** 3, dtype=np.float32) * np.float32(2.0 ** 36)
+        for q in (k, k + 1):
+            u[int(B.offsets[q]):int(B.offsets[q]) + v.size] = v
+    B.set_fields(u)
+    B.step(1)
+    info, got = B.member_info(), B.get_fields()
+    assert np.all(info["status"] == 0) and np.all(info["rel"] <= 1e-8), info
+    for k in (0, 2):
+        assert np.array_equal(B.member(got, k), B.member(got, k + 1))
+    B.close()
