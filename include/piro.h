@@ -405,6 +405,11 @@ int piro_be_create_stencil(int nx, int ny, int nz, const int32_t *rowptr, const 
  * variable PIRO_BE_PERSISTENT, read at creation, forces kind <= 1 ("0") or
  * keeps kind 2 instead of 3 ("g"). */
 int piro_be_inner_operator(piro_be_solver *s, int *kind);
+/* The kernels a plain solve and a learned or flexible sweep's Jacobi iterations
+ * take: 0 launches per phase, 1 one launch with the vectors in global memory,
+ * 2 one launch with p, d, q in shared memory, 3 one launch with the whole state
+ * on chip (inner operator kind 3 is 2 or 3). */
+int piro_be_forms(piro_be_solver *s, int *plain, int *flexible);
 /* Algorithmic bytes moved by the persistent launches counted in
  * piro_be_kernel_stats (since its last reset). */
 int piro_be_persistent_bytes(piro_be_solver *s, double *bytes);

@@ -100,6 +100,7 @@ SIGNATURES = {
     "piro_be_create": (i32, [i32, i32, i32, vp, vp, vp, vp, vp, C.POINTER(vp)]),
     "piro_be_create_stencil": (i32, [i32, i32, i32, vp, vp, vp, vp, f32, f32, vp, C.POINTER(vp)]),
     "piro_be_inner_operator": (i32, [vp, pint]),
+    "piro_be_forms": (i32, [vp, pint, pint]),
     "piro_be_persistent_bytes": (i32, [vp, C.POINTER(C.c_double)]),
     "piro_be_solve": (i32, [vp, vp, vp, f64, i32, i32, C.POINTER(BeInfo)]),
     "piro_be_solution_f64": (i32, [vp, C.POINTER(vp)]),

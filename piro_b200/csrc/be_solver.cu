@@ -2123,14 +2123,50 @@ extern "C" int piro_be_pc_stats(piro_be_solver *s, int reset, long long *applies
     return PIRO_OK;
 }
 
+// The forms of the solve, chosen once here for the launches and for the query.
+enum : int { kFormLaunches = 0, kFormGlobal = 1, kFormShared = 2, kFormChip = 3 };
+
+// float4 groups can be used on every vector (the work vectors are 256-byte aligned)
+static bool be_vec(const piro_be_solver *s)
+{
+    const bool al16 = ((reinterpret_cast<uintptr_t>(s->alpha) | reinterpret_cast<uintptr_t>(s->dinv)) & 15) == 0;
+    return al16 && s->N % 4 == 0 && s->nx % 4 == 0;
+}
+
+static int be_plain_form(const piro_be_solver *s)
+{
+    if (!s->persist) return kFormLaunches;
+    if (s->rc_team > 0) return kFormChip;
+    return s->res_cells > 0 && be_vec(s) ? kFormShared : kFormGlobal;
+}
+
+// A learned or flexible sweep's Jacobi iterations: on chip, but for runs of more
+// than five groups per thread where k_fcg_persistent keeps its vectors on chip as
+// well.  Solves on B200, on chip / not: 64^3 617 / 742 us, 87 x 64 x 75 741 / 1002,
+// 112^3 (5 groups) 867 / 934, 120^3 (6) 1018 / 1005, 128^3 (7) 1152 / 1142; off the
+// float4 forms 125 x 127 x 126 (7) 1085 / 1731.
+static int be_flexible_form(const piro_be_solver *s)
+{
+    if (!s->persist) return kFormLaunches;
+    const bool beside = s->fcg_res && s->res_cells > 0 && s->nx % 4 == 0 && s->rc_problem.groups > 5 * kRcThreads;
+    if (s->rc_team > 0 && !beside) return kFormChip;
+    if (s->grid_fp == 0) return kFormLaunches;
+    return s->fcg_res && s->res_cells > 0 && be_vec(s) ? kFormShared : kFormGlobal;
+}
+
+extern "C" int piro_be_forms(piro_be_solver *s, int *plain, int *flexible)
+{
+    PIRO_ARG(s && plain && flexible, "piro_be_forms: bad arguments");
+    *plain = be_plain_form(s);
+    *flexible = be_flexible_form(s);
+    return PIRO_OK;
+}
+
 extern "C" int piro_be_inner_operator(piro_be_solver *s, int *kind)
 {
     PIRO_ARG(s && kind, "piro_be_inner_operator: bad arguments");
     *kind = s->op_mf ? (s->persist ? 2 : 1) : 0;
-    if (*kind == 2) {  // the resident variant, when its float4 paths are usable at solve time
-        const bool al16 = ((reinterpret_cast<uintptr_t>(s->alpha) | reinterpret_cast<uintptr_t>(s->dinv)) & 15) == 0;
-        if (s->rc_team > 0 || (s->res_cells > 0 && al16 && s->N % 4 == 0 && s->nx % 4 == 0)) *kind = 3;
-    }
+    if (*kind == 2 && be_plain_form(s) != kFormGlobal) *kind = 3;
     return PIRO_OK;
 }
 
@@ -2188,7 +2224,8 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
         const bool al16 = ((reinterpret_cast<uintptr_t>(s->alpha) | reinterpret_cast<uintptr_t>(s->dinv)) & 15) == 0;
         P.vec_b = (N % 4 == 0) && al16;
         P.vec_a = P.vec_b && (s->nx % 4 == 0);
-        const bool res = s->res_cells > 0 && P.vec_a;
+        const int form = be_plain_form(s);
+        const bool res = form == kFormShared;
         P.own_cells = res ? s->res_cells : 0;
         void *args[] = {&P};
         RcProblem Q = s->rc_problem;
@@ -2197,7 +2234,7 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
         void *rargs[] = {&Q, &epoch, &slots, &s->st, &P.spin_limit};
         PIRO_CUDA(cudaMemsetAsync(s->st, 0, sizeof(DevState), st));
         PIRO_CUDA(cudaEventRecord(s->pev0, st));
-        if (s->rc_team > 0) {
+        if (form == kFormChip) {
             Q.alpha = s->alpha;
             Q.mdt = s->mdt;
             Q.vself = s->vself;
@@ -2302,14 +2339,8 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
         while (true) {
             const bool with_net = net_iters;
             net_iters = false;
-            // The rest of the sweep on chip, but for runs of more than five groups per
-            // thread where k_fcg_persistent keeps its vectors on chip as well.  Solves
-            // on B200, on chip / not: 64^3 617 / 742 us, 87 x 64 x 75 741 / 1002, 112^3
-            // (5 groups) 867 / 934, 120^3 (6) 1018 / 1005, 128^3 (7) 1152 / 1142; off
-            // the float4 forms 125 x 127 x 126 (7) 1085 / 1731.
-            const bool beside = s->fcg_res && s->res_cells > 0 && s->nx % 4 == 0 && s->rc_problem.groups > 5 * kRcThreads;
-            const bool on_chip = learned && !with_net && s->persist && s->rc_team > 0 && !beside;
-            if (on_chip && !s->rc_fcg) {
+            const int form = learned && !with_net ? be_flexible_form(s) : kFormLaunches;
+            if (form == kFormChip && !s->rc_fcg) {
                 // one CTA per SM, as k_be_resident: the same threads, registers and shared memory at most
                 const RcProblem &rp = s->rc_problem;
                 const void *fcg = rp.wide_s ? fcg_resident_kernel<true>(rp.groups, rp.ax != nullptr)
@@ -2317,7 +2348,7 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
                 PIRO_CUDA(cudaFuncSetAttribute(fcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRcSmemMax));
                 s->rc_fcg = fcg;
             }
-            if (on_chip) {
+            if (form == kFormChip) {
                 RcProblem Q = s->rc_problem;
                 Q.alpha = s->alpha;
                 Q.mdt = s->mdt;
@@ -2348,7 +2379,7 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
                 seen = s->h_st->iters;
                 break;
             }
-            if (learned && !with_net && s->persist && s->grid_fp > 0) {
+            if (form != kFormLaunches) {
                 // the same in one cooperative launch with two grid barriers per iteration
                 PArgs F{};
                 F.g = GridDiv(s->nx, s->ny, s->nz);
@@ -2367,13 +2398,10 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
                 F.partials = s->partials;
                 F.st = s->st;
                 F.spin_limit = wait_limit(1ll << 22);
-                const uintptr_t al = reinterpret_cast<uintptr_t>(s->alpha) | reinterpret_cast<uintptr_t>(s->dinv) |
-                                     reinterpret_cast<uintptr_t>(s->r) | reinterpret_cast<uintptr_t>(s->z) |
-                                     reinterpret_cast<uintptr_t>(s->q) | reinterpret_cast<uintptr_t>(s->d) |
-                                     reinterpret_cast<uintptr_t>(s->p[0]) | reinterpret_cast<uintptr_t>(s->p[1]);
-                F.vec_b = (N % 4 == 0) && (al & 15) == 0;
-                F.vec_a = F.vec_b && (s->nx % 4 == 0);
-                const bool res = s->fcg_res && s->res_cells > 0 && F.vec_a;
+                const bool al16 = ((reinterpret_cast<uintptr_t>(s->alpha) | reinterpret_cast<uintptr_t>(s->dinv)) & 15) == 0;
+                F.vec_b = N % 4 == 0 && al16;
+                F.vec_a = be_vec(s);
+                const bool res = form == kFormShared;
                 F.own_cells = res ? s->res_cells : 0;
                 void *fargs[] = {&F};
                 PIRO_CUDA(cudaMemsetAsync(&s->st->bar_count, 0, 2 * sizeof(unsigned) + sizeof(int), st));

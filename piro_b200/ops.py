@@ -388,6 +388,16 @@ class BESolver:
         check(lib().piro_be_inner_operator(self.h, C.byref(k)), "piro_be_inner_operator")
         return {2: "global", 3: "resident"}.get(k.value)
 
+    @property
+    def forms(self):
+        """Of a plain solve and of a flexible sweep's Jacobi iterations: 'launches' (one
+        per phase), or one launch with the vectors in 'global' memory, in 'shared'
+        memory, or with the whole state on 'chip'."""
+        a, b = C.c_int(), C.c_int()
+        check(lib().piro_be_forms(self.h, C.byref(a), C.byref(b)), "piro_be_forms")
+        names = ["launches", "global", "shared", "chip"]
+        return names[a.value], names[b.value]
+
     def persistent_bytes(self):
         v = C.c_double()
         check(lib().piro_be_persistent_bytes(self.h, C.byref(v)), "piro_be_persistent_bytes")
