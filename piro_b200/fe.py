@@ -7,6 +7,8 @@ launch.  The per-step launches can also be captured once in a CUDA graph and
 replayed (graph=True, capture)."""
 from __future__ import annotations
 
+import operator
+
 import torch
 
 from . import ops
@@ -41,7 +43,10 @@ class _Loop:
         torch.cuda.current_stream().wait_stream(stream)
         self._graph = g
 
+        memD = self.memD
+
         def replay(pairs: int) -> torch.Tensor:
+            assert memD is not None  # what the graph reads, whatever runs come between
             bufs[0].copy_(u0)
             for _ in range(pairs):
                 g.replay()
@@ -51,9 +56,11 @@ class _Loop:
 
     def run(self, u0: torch.Tensor, steps: int, graph: bool = False) -> torch.Tensor:
         if not graph:
-            u0 = u0.contiguous()
+            steps = max(operator.index(steps), 0)
+            # a clone makes a slice contiguous, and leaves a permuted field to be refused
+            self.memD = u0 if u0.is_contiguous() else u0.clone()
             bufs = [torch.empty_like(u0), torch.empty_like(u0)]
-            return ops.csr_fe_run_bc(self.nx, self.ny, self.nz, self.A, self.dt, u0, u0, *bufs, steps)
+            return ops.csr_fe_run_bc(self.nx, self.ny, self.nz, self.A, self.dt, self.memD, self.memD, *bufs, steps)
         self._setup_bc(u0)
         bufs = [u0.clone(), torch.empty_like(u0)]
         # two steps per graph (buffers ping-pong), replayed steps//2 times

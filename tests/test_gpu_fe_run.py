@@ -45,3 +45,30 @@ def test_run_equals_steps(cuda, n, steps, kind):
         ops.csr_fe_step_bc(nx, ny, nz, A, 0.03, u, bc, out)
         u, out = out, u
     assert f32_bits_equal(got.cpu().numpy(), u.cpu().numpy())
+
+
+@pytest.mark.parametrize("n", [(12, 10, 9), (40, 36, 33)])  # one cluster, a launch per step
+def test_run_takes_what_the_step_loop_took(cuda, n):
+    """Slices and step counts of zero and below; a permuted field and a fraction of a
+    step refused; the face values kept for single steps."""
+    import torch
+    from piro_b200 import fe
+    N = n[0] * n[1] * n[2]
+    run = fe.FeRunner(*n, torch.full((N,), 0.01, device="cuda"), 3.0)
+    wide = torch.rand(2 * N, device="cuda")
+    u = wide[::2].clone()
+    want = run.run(u, 3, graph=True)
+    assert torch.equal(run.run(wide[::2], 3), want)
+    for steps in (0, -2):
+        got = run.run(u, steps)
+        assert torch.equal(got, u) and got.data_ptr() != u.data_ptr()
+    with pytest.raises(TypeError):
+        run.run(u, 2.0)
+    with pytest.raises(ValueError):
+        run.run(u.reshape(n).permute(2, 1, 0), 3)
+    v = torch.rand_like(u)
+    out = run.run(v, 1)
+    assert torch.equal(run.memD, v)
+    one = torch.empty_like(v)
+    run._step(v, one)
+    assert torch.equal(one, out)
