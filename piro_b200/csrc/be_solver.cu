@@ -1890,10 +1890,14 @@ static int be_setup_persistent(piro_be_solver *s, bool allow_resident)
             int per_sm_rc = 0;
             s->rc_smem = rc_smem(rp, false, stream);
             PIRO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rc, kern, kRcThreads, s->rc_smem));
-            if (per_sm_rc >= 1) {
-                const size_t ex = rc_exchange_bytes(s->nx, s->ny, s->nz), comm = 256 + rc_slot_bytes(team);
-                s->rc_bytes = comm + ex;
-                PIRO_CUDA(cudaMalloc(&s->rc_mem, s->rc_bytes + (stream ? ex / 2 : 0)));
+            const size_t ex = rc_exchange_bytes(s->nx, s->ny, s->nz), comm = 256 + rc_slot_bytes(team);
+            s->rc_bytes = comm + ex;
+            // without the memory for it the other forms solve as well
+            if (per_sm_rc >= 1 && cudaMalloc(&s->rc_mem, s->rc_bytes + (stream ? ex / 2 : 0)) != cudaSuccess) {
+                (void)cudaGetLastError();
+                s->rc_mem = nullptr;
+            }
+            if (s->rc_mem) {
                 PIRO_CUDA(cudaMemsetAsync(s->rc_mem, 0, s->rc_bytes, s->stream));
                 rp.zx = reinterpret_cast<uint4 *>(s->rc_mem + comm);
                 rp.ax = stream ? reinterpret_cast<float4 *>(s->rc_mem + s->rc_bytes) : nullptr;
