@@ -966,7 +966,8 @@ static void batch_free_groups(piro_batch *s)
 // teams end sooner, so a few common factors are tried on the list schedule
 // below and the shortest is taken.  Cycles of an iteration from the 128^3
 // solve's phases (B200): 8000 for a team's waits (3000 for one CTA's), 3.5 per
-// group of a CTA.  Returns PIRO_OK with d_rjobs unset if a member does not fit.
+// group of a CTA.  Returns PIRO_OK with d_rjobs unset if a member does not fit, or
+// the exchange buffers in what device memory is left.
 static int batch_resident_setup(piro_batch *s)
 {
     int dev = 0;
@@ -1074,7 +1075,12 @@ static int batch_resident_setup(piro_batch *s)
     }
     ptr[C] = (int)list.size();
     cudaError_t e = cudaMalloc(&s->r_mem, bytes > 0 ? bytes : 256);
-    if (e == cudaSuccess) e = cudaMemset(s->r_mem, 0, bytes > 0 ? bytes : 256);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        s->r_mem = nullptr;
+        return PIRO_OK;
+    }
+    e = cudaMemset(s->r_mem, 0, bytes > 0 ? bytes : 256);
     for (RJob &J : jobs)
         if (J.gsize > 1) {
             J.epoch = reinterpret_cast<unsigned long long *>(s->r_mem + reinterpret_cast<size_t>(J.epoch));

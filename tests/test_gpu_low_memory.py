@@ -1,6 +1,7 @@
 """With device memory for the older forms but not for the on-chip form's exchange
-buffers, solvers are created all the same and solve in an older form.
+buffers, solvers and batches are created all the same and solve in an older form.
 The rest of the device memory is held by one allocation meanwhile."""
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,32 @@ def test_be_solver_without_the_exchange_buffer(cuda, monkeypatch):
     with _Full(torch, free - used + 10 * MIB):  # the exchange buffer and alpha take 24 MB
         assert run(x)[1] == "shared"
     assert float((x - want).abs().max()) <= 1e-6 * float(want.abs().max())
+
+
+def test_batch_without_the_exchange_buffer(cuda):
+    import torch
+    from piro_b200 import ops
+    n = np.array([127], np.int32)  # 16 MB
+    alpha, dt = np.array([0.01], np.float32), np.array([830.0], np.float32)
+    u = np.random.default_rng(0).random(int(n[0]) ** 3, dtype=np.float32)
+    got = []
+    for low in (False, True):
+        B = ops.Batch(n, alpha, dt, np.ones(1, np.int32))
+        u0 = np.zeros(B.total, np.float32)
+        u0[:u.size] = u
+        if low:
+            B.set_schedule(False, 4)
+            B.set_fields(u0)
+            B.step(1)
+            with _Full(torch, 8 * MIB):
+                B.set_schedule(True, 2)
+                B.set_fields(u0)
+                B.step(1)
+        else:
+            B.set_schedule(True, 2)
+            B.set_fields(u0)
+            B.step(1)
+        assert np.all(B.member_info()["rel"] <= 1e-8)
+        got.append(B.member(B.get_fields(), 0))
+        B.close()
+    assert np.abs(got[0] - got[1]).max() <= 1e-6 * np.abs(got[0]).max()
