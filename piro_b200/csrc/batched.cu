@@ -1675,7 +1675,10 @@ extern "C" int piro_batch_set_schedule(piro_batch *s, int grouped, int blocks_pe
     batch_drop_graph(s);
     if (grouped) {
         int rc = batch_groups_setup(s, blocks_per_sm);
-        if (rc) return rc;
+        if (rc) {
+            s->grouped = 0;  // the jobs of the schedule before are gone
+            return rc;
+        }
     } else {
         int rc = batch_tiles(s, s->tile, blocks_per_sm);
         if (rc) return rc;
