@@ -360,11 +360,11 @@ __global__ void __launch_bounds__(256) k_conv_bwd_w(GridDiv g, int64_t N, int B,
 // threads per value add a stretch of the blocks each, 16 loads at a time, and the
 // first of them adds the stretches.  Bound by latency: 148 partials of 6912 values
 // take 5 us; one thread per value took 17 with 32 loads at a time and 22 with
-// four (B200).
+// four (B200).  The loads go to L2: the kernel before may still write the partials
+// while this one sets up, which rules out the path for data read only.
 constexpr int kRedSegs = 8;
 
-__global__ void __launch_bounds__(32 * kRedSegs) k_reduce_partials(const float *__restrict__ partials, int nblocks, int P,
-                                                                   float *__restrict__ out)
+__global__ void __launch_bounds__(32 * kRedSegs) k_reduce_partials(const float *partials, int nblocks, int P, float *out)
 {
     __shared__ double s_seg[kRedSegs][32];
     tc::grid_launch_next();
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(32 * kRedSegs) k_reduce_partials(const float *
         for (int k0 = b0; k0 < b1; k0 += 16) {
             float v[16];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = __ldg(partials + (int64_t)(k0 + k < b1 ? k0 + k : b1 - 1) * P + p);
+            for (int k = 0; k < 16; ++k) v[k] = __ldcg(partials + (int64_t)(k0 + k < b1 ? k0 + k : b1 - 1) * P + p);
 #pragma unroll
             for (int k = 0; k < 16; ++k) s += k0 + k < b1 ? (double)v[k] : 0.0;  // + 0: s is never -0
         }
