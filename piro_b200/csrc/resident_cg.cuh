@@ -168,10 +168,11 @@ inline RcProblem rc_geometry(int nx, int ny, int nz, int size)
     P.fh = FastDiv((uint32_t)P.h);
     P.fhl = FastDiv((uint32_t)P.hlast);
     P.fly = FastDiv((uint32_t)ny);
-    // the largest run, and the most neighbour lines outside a run
+    // the largest run, and (a walk over the lines) the most neighbour lines outside a
+    // run, which a grid too large for the chip needs no count of
     P.groups = (int)(cdiv(P.lines, size) * P.gx);
     P.halo = 0;
-    if (size > 1) {
+    if (size > 1 && P.groups <= kRcGroups) {
         int l = 0;
         for (int r = 0, st = 0, y = 0, zz = 0; r < size; ++r) {
             const int l0 = l, l1 = (int)((int64_t)P.lines * (r + 1) / size);
