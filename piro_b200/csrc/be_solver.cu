@@ -2270,11 +2270,16 @@ extern "C" int piro_be_solve(piro_be_solver *s, const float *b, float *x, double
         if (cudaEventElapsedTime(&ms, s->pev0, s->pev1) == cudaSuccess) {
             s->persist_ms += ms;
             s->persist_launches += 1;
-            // algorithmic bytes: P0 32, residual sweep 32 + update 24, CG iteration 8 (phase A: z, alpha)
-            // + 12 (phase B: z, alpha in, z out) bytes per cell (k_be_persistent with p, d, q on chip; k_be_resident
-            // keeps z there as well)
-            const double n = (double)N;
-            s->persist_bytes += n * (32.0 + 56.0 * (s->h_st->p_outer + 1) + 20.0 * s->h_st->p_inner + 8.0);
+            // algorithmic bytes per cell.  On chip: alpha for D 4, a residual 8 and after
+            // the first 8 more (b, alpha; x64), a correction 16 (x64 in and out), the
+            // result 12; alpha again in every iteration where it is streamed.  Else: P0 32, a
+            // residual 32, a correction 24, an iteration 8 (z, alpha) + 12 (z, alpha in,
+            // z out), the result 8.
+            const double n = (double)N, outer = s->h_st->p_outer, inner = s->h_st->p_inner;
+            if (form == kFormChip)
+                s->persist_bytes += n * (24.0 + 32.0 * outer + (Q.ax ? 4.0 + 4.0 * inner : 0.0));
+            else
+                s->persist_bytes += n * (32.0 + 56.0 * (outer + 1) + 20.0 * inner + 8.0);
         } else {
             (void)cudaGetLastError();
         }

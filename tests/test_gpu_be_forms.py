@@ -67,3 +67,17 @@ def test_flexible_forms(cuda, n, env, form, with_net, monkeypatch):
         got[e], info = _solve(s, b)
         assert info.fallbacks == 0
     assert np.abs(got[env] - got["0"]).max() <= 1e-6 * np.abs(got["0"]).max()
+
+
+@pytest.mark.parametrize("n", [(40, 32, 24), (128, 126, 127)])  # alpha on chip, alpha streamed
+def test_bytes_of_the_on_chip_solve(cuda, n, monkeypatch):
+    s, b = _solver(n, monkeypatch)
+    import torch
+    x = torch.empty_like(b)
+    s.solve(b, x)
+    s.kernel_stats(reset=True)
+    info = s.solve(b, x)
+    N = b.numel()
+    want = 24 + 32 * info.outer_iterations + (4 + 4 * info.inner_iterations if n[0] == 128 else 0)
+    assert s.persistent_bytes() == want * N
+    s.close()
