@@ -1606,7 +1606,8 @@ extern "C" int piro_batch_autotune(piro_batch *s, double rtol, int *tile_out, in
 {
     PIRO_ARG(s && rtol > 0.0, "piro_batch_autotune: bad arguments");
     s->rtol = rtol;
-    s->grouped = 0;  // the lockstep candidates first
+    batch_drop_graph(s);  // it holds the lists that the candidates free
+    s->grouped = 0;       // the lockstep candidates first
     const int tiles[] = {2048, 4096, 8192, 16384};
     const int bps[] = {1, 2, 4, 6, 8};
     double best = INFINITY;
@@ -1652,7 +1653,6 @@ extern "C" int piro_batch_autotune(piro_batch *s, double rtol, int *tile_out, in
     } else {
         batch_free_groups(s);
     }
-    batch_drop_graph(s);
     if (!std::isfinite(best)) {
         set_error("piro_batch_autotune: grid barrier timed out in every candidate");
         return PIRO_ERR_CUDA;
