@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(256) k_lupb_update(int64_t N, int64_t bw, int6
 //
 // Every element receives the operations of the column launches in their
 // order: the band, the multipliers and the pivots are the same bits.  At 24^3
-// (864 panels of 592 rows) 23.3 ms, against 74.6 by three launches per panel
+// (864 panels of 592 rows) 23.1 ms, against 74.6 by three launches per panel
 // with the panel in shared memory and three barriers a step; 12^3 2.1 against
 // 7.1, 24 x 24 x 6 5.9 against 18.3 (B200).  Block 0 per panel, in thousands of
 // cycles: the steps 35, Lp out 5, the next columns' pivot rows

@@ -493,9 +493,9 @@ __global__ void k_scale_add(int64_t n, float dt, const float *acc, const float *
 
 // HT lookup with linear probing (SpMVHT.cl:1-20) from slot h on; bounded by
 // the table's length.  Four slots at a time: a warp walks as far as its longest
-// chain, and a slot by itself costs a load's latency.  With the staged step at
-// 256^3 (1178 us; 64^3 35): one slot at a time 1294 (54), three 1162 (38), eight
-// 1248 (37) (B200).
+// chain, and a slot by itself costs a load's latency.  The staged step at 256^3
+// (and 64^3), one run on a B200: four 1178 us (35), one slot at a time 1294 (54),
+// three 1162 (38), eight 1248 (37); 1170 to 1280 over boxes.
 template <typename I>
 __device__ __forceinline__ float ht_get_from(int64_t key, I h, const int64_t *__restrict__ keys,
                                              const float *__restrict__ vals, I ts)
